@@ -133,7 +133,9 @@ typedef struct {
    checked against the list.  The pair set and the FP32 forces are identical
    to CELLS.  AUTO starts with CELLS and, at the first rdgpu_step of >= 4 x
    graph_steps steps, times CELLS and LIST at skins of 0.1 .. 0.5 x rc_max on
-   the handle's particles and keeps the fastest.  Every energy, force, digest
+   the handle's particles and keeps the fastest; the pair-list steps of an AUTO
+   handle run many to a kernel launch, those of a LIST handle launch by launch
+   in captured graphs.  Every energy, force, digest
    or RDF evaluation in LIST mode re-sorts and rebuilds the list (one build in
    list_builds).                                                                */
 #define RDGPU_NB_AUTO  0

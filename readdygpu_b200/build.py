@@ -37,7 +37,7 @@ def _stale(out, deps):
 
 def build_engine(force=False):
     out = os.path.join(HERE, "libreaddy_b200.so")
-    deps = [os.path.join(CSRC, f) for f in ("engine.cu", "engine_kernels.cuh", "engine_device.cuh", "rdf_noalloc.cu")]
+    deps = [os.path.join(CSRC, f) for f in ("engine.cu", "engine_kernels.cuh", "engine_run.cuh", "engine_device.cuh", "rdf_noalloc.cu")]
     deps.append(os.path.join(ROOT, "include", "readdy_b200.h"))
     if force or _stale(out, deps):
         _run([NVCC] + ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-shared",

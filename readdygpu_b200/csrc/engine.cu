@@ -3,9 +3,10 @@
 //
 // Replaces the reference's CudaSimulation host wrapper
 // (lib/ReaDDyGPU_Cpp/CudaKernels/CudaSimulation.cu:138-626, 2309-2476):
-// device state, cell binning, per-step launches.  One stream per handle; the
-// steps of rdgpu_step are replayed from a captured CUDA graph of
-// step_kernel -> scan_tiles -> scan_apply -> scatter per step.
+// device state, cell binning, per-step launches.  One stream per handle.  The
+// pair-list steps of an AUTO handle run in one launch per rdgpu_step call
+// (list_run_kernel); the others are replayed from captured CUDA graphs, with
+// step_kernel -> scan_tiles -> scan_apply -> scatter per step of the cell walk.
 #include <algorithm>
 #include <map>
 #include <cmath>
@@ -16,6 +17,7 @@
 
 #include "../../include/readdy_b200.h"
 #include "engine_kernels.cuh"
+#include "engine_run.cuh"
 
 using namespace rdgpu;
 
@@ -36,9 +38,19 @@ constexpr long long kHotDiv = 300;
 // 128, 256 and 1019 blocks measured slower per step on config 4)
 constexpr int kCheckBlock = 256;
 constexpr int kCheckBlocks = 512;
+// steps of one list_run_kernel launch, at most
+constexpr long long kRunSteps = 1024;
 }  // namespace
 
 std::string& rdgpu_global_error() { return g_create_error; }
+
+// what a handle's kernels and copies report to the host (page-locked)
+struct Pinned {
+    int err;
+    long long step;
+    ListCtl ctl;
+    RunOut run;
+};
 
 // the opaque handle type of the C ABI
 struct rdgpu_engine {
@@ -103,7 +115,8 @@ struct rdgpu_engine {
     double* part_d = nullptr;            // partial sums of the typed reductions
     long long* off_d = nullptr;          // particle offsets of the systems (n_systems + 1)
     long long* pcnt_d = nullptr;
-    int* pinned_err = nullptr;
+    Pinned* pinned = nullptr;
+    int* pinned_err = nullptr;           // its parts
     long long* pinned_step = nullptr;
     long long step_h = 0;
     // RDF accumulator
@@ -133,6 +146,12 @@ struct rdgpu_engine {
     bool tuned = false;
     bool tuning = false;                 // inside tune(): its trials do not re-tune
     bool retune = false;                 // the lists outgrew their capacity: tune again
+    RunCtl* run_ctl = nullptr;           // list_run_kernel: the control words of this launch and the next
+    int run_k = 0;                       // which of the two the next launch takes
+    RunOut* run_out = nullptr;           // its outcome (page-locked)
+    int* run_tsum = nullptr;             // its scan's tile sums
+    long long run_tsum_n = 0;
+    int sm_count = 0;
     ListCtl* ctl = nullptr;
     ListCtl* pinned_ctl = nullptr;
     int nbuild_h = 0;
@@ -713,7 +732,7 @@ int ensure_list(Engine* E, int cap, bool wide)
     const long long groups = wide ? cap / 4 : cap / 8;
     CK(cudaMalloc(&E->nbr, (size_t)groups * stride * sizeof(int4)));
     CK(cudaMalloc(&E->head, stride * sizeof(uint2)));
-    CK(cudaMalloc(&E->hot, kHotMax * sizeof(int)));
+    CK(cudaMalloc(&E->hot, 2 * kHotMax * sizeof(int)));   // two steps' (list_run_kernel)
     E->list_cap = cap;
     E->list_stride = stride;
     E->list_wide = wide;
@@ -823,12 +842,24 @@ void launch_list_step_kernel_w(Engine* E, const Args<R>& a, const ListArgs<R>& v
         list_step_kernel<R, false, false, kListBlock, NARROW><<<grid, kListBlock, 0, E->stream>>>(a, v);
 }
 
+// every axis of every system is periodic
+bool all_periodic(const Engine* E)
+{
+    for (int s = 0; s < E->nsys; ++s)
+        for (int q = 0; q < 3; ++q)
+            if (!E->sys_h[s].per[q]) return false;
+    return true;
+}
+
+// Pair-list steps of an AUTO handle run in one launch (list_run_kernel); a
+// handle that asked for RDGPU_NB_LIST steps launch by launch, as its options
+// say, in captured graphs.
+bool run_in_one(const Engine* E) { return E->nb_req == RDGPU_NB_AUTO && E->graph_steps > 0; }
+
 template <class R> void launch_list_step_kernel(Engine* E, const Args<R>& a, const ListArgs<R>& v)
 {
     const int grid = (int)((E->npart_tot + kListBlock - 1) / kListBlock);
-    bool allper = true;
-    for (int s = 0; s < E->nsys; ++s)
-        for (int q = 0; q < 3; ++q) allper = allper && E->sys_h[s].per[q];
+    const bool allper = all_periodic(E);
     if (v.narrow)
         launch_list_step_kernel_w<R, true>(E, a, v, grid, allper);
     else
@@ -987,8 +1018,115 @@ template <class R> int capture_list_graph(Engine* E, int n, cudaGraphExec_t* out
     return RDGPU_OK;
 }
 
+// list_run_kernel with as many threads per particle tile as the GPU has room
+// for: up to 4 tiles per SM, one block of 4 warps on as many SMs as it takes
+// (the fewer warps an SM runs, the sooner each is done); up to a block per
+// SM, all SMs with the warps their tiles need; beyond that, all blocks that
+// fit.  Blocks of 128 or 256 threads on the same number of warps measured 15
+// to 35 % slower at 250,000 particles (more arrivals at the barrier, shares
+// that differ more).
+template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E, RunArgs<R>& p)
+{
+    using S = RunShape<R, HREP, ALLPER>;
+    const void* f = (const void*)list_run_kernel<R, HREP, ALLPER, NARROW>;
+    const long long tiles = (E->npart_tot + 31) / 32;
+    const int sms = E->sm_count;
+    int block = S::BLOCK, grid = 1;
+    if (tiles <= 4LL * sms) {
+        block = 128;
+        grid = (int)((tiles + 3) / 4);
+    } else if (tiles <= (long long)sms * (S::BLOCK / 32)) {
+        block = 32 * (int)((tiles + sms - 1) / sms);
+        grid = sms;
+    } else {
+        constexpr int wpb = S::BLOCK / 32;
+        grid = (int)std::min<long long>((long long)sms * S::PER_SM, (tiles + wpb - 1) / wpb);
+    }
+    void* args[] = {&p};
+    CK(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(block), args, 0, E->stream));
+    ++E->launches;
+    return RDGPU_OK;
+}
+
+template <class R, bool NARROW> int launch_run_w(Engine* E, RunArgs<R>& p, bool allper)
+{
+    if (E->hrep) return allper ? launch_run<R, true, true, NARROW>(E, p) : launch_run<R, true, false, NARROW>(E, p);
+    return allper ? launch_run<R, false, true, NARROW>(E, p) : launch_run<R, false, false, NARROW>(E, p);
+}
+
+// one launch of up to n pair-list steps from step step_h; waits for it
+template <class R> int run_steps(Engine* E, int n)
+{
+    // scan tiles of the smallest block
+    const long long nt = E->ncells_tot / (128 * RUN_SCAN_PER) + 2;
+    if (nt > E->run_tsum_n) {
+        dfree(E->run_tsum);
+        E->run_tsum_n = 0;
+        CK(cudaMalloc(&E->run_tsum, nt * sizeof(int)));
+        E->run_tsum_n = nt;
+    }
+    RunArgs<R> p;
+    memset(&p, 0, sizeof(p));
+    p.a = make_args<R>(E);
+    p.v = make_list_args<R>(E, true);
+    p.ctl = E->run_ctl + E->run_k;
+    p.next = E->run_ctl + (E->run_k ^ 1);
+    p.out = E->run_out;
+    p.tile_sum = E->run_tsum;
+    p.ncells = E->ncells_tot;
+    p.t0 = E->step_h;
+    p.nsteps = n;
+    p.sel0 = E->cur;
+    const int rc = p.v.narrow ? launch_run_w<R, true>(E, p, all_periodic(E)) : launch_run_w<R, false>(E, p, all_periodic(E));
+    if (rc) return rc;
+    E->run_k ^= 1;
+    CK(cudaStreamSynchronize(E->stream));
+    return RDGPU_OK;
+}
+
+// do_steps_list by list_run_kernel
+template <class R> int do_steps_run(Engine* E, long long nsteps)
+{
+    const long long target = E->step_h + nsteps;
+    while (E->step_h < target) {
+        int rc = run_steps<R>(E, (int)std::min<long long>(target - E->step_h, kRunSteps));
+        if (rc) return rc;
+        const RunOut o = *E->run_out;
+        if (o.dead) {
+            E->part_off.clear();
+            return fail(E, RDGPU_ERR_CUDA, "a grid barrier of the step kernel timed out");
+        }
+        E->step_h = o.t;
+        E->nbuild_h += o.builds;
+        set_cur(E, o.sel);
+        if (o.err == 0) continue;
+        // the input of step step_h is intact in buffer cur
+        if ((o.err & ~(EF_LISTOVF | EF_LISTWIDE)) == 0) {
+            E->pinned_ctl->maxcnt = o.maxcnt;
+            rc = ensure_list_after(E, o.err);
+            if (rc) return rc;
+            rc = resort<R>(E, true);
+            if (rc) return rc;
+            // the particles gathered into denser clusters than the tuner saw:
+            // an AUTO handle times its options again on the new state
+            if ((o.err & EF_LISTOVF) && E->nb_req == RDGPU_NB_AUTO && !E->tuning) {
+                E->retune = true;
+                return RDGPU_OK_CONTINUE;
+            }
+            continue;
+        }
+        rc = prepare_step_state(E, o.t);
+        if (rc) return rc;
+        if (o.err & EF_NONFINITE)
+            return fail(E, RDGPU_ERR_NONFINITE, "a particle position became non-finite at step " + std::to_string(o.t));
+        return fail(E, RDGPU_ERR_JUMP, "a particle moved more than a box length at step " + std::to_string(o.t));
+    }
+    return RDGPU_OK;
+}
+
 template <class R> int do_steps_list(Engine* E, long long nsteps, const double* noise_d)
 {
+    if (run_in_one(E) && !noise_d) return do_steps_run<R>(E, nsteps);
     const long long target = E->step_h + nsteps;
     while (E->step_h < target) {
         long long remaining = target - E->step_h;
@@ -1138,6 +1276,7 @@ template <class R> int tune(Engine* E)
 template <class R> int prepare_graph(Engine* E)
 {
     if (E->graph_steps <= 0) return RDGPU_OK;
+    if (E->nb_mode == RDGPU_NB_LIST && run_in_one(E)) return RDGPU_OK;   // nothing to capture
     std::vector<int> sizes = {E->graph_steps};
     for (int p = 1; p < E->graph_steps; p <<= 1) sizes.push_back(p);
     for (int n : sizes) {
@@ -2084,9 +2223,13 @@ int create_impl(const rdgpu_system_desc* desc, int nsys, const rdgpu_box* boxes,
         cudaMalloc(&E->part_d, (RDGPU_MAX_TYPES + 1) * kSumParts * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&E->off_d, (nsys + 1) * sizeof(long long)) != cudaSuccess ||
         cudaMalloc(&E->pcnt_d, (RDGPU_MAX_TYPES + 1) * kSumParts * sizeof(long long)) != cudaSuccess ||
-        cudaMallocHost(&E->pinned_err, sizeof(int)) != cudaSuccess ||
-        cudaMallocHost(&E->pinned_step, sizeof(long long)) != cudaSuccess)
+        cudaMallocHost(&E->pinned, sizeof(Pinned)) != cudaSuccess ||
+        cudaDeviceGetAttribute(&E->sm_count, cudaDevAttrMultiProcessorCount, o.device) != cudaSuccess)
         return bail(RDGPU_ERR_NOMEM, "device allocation failed");
+    E->pinned_err = &E->pinned->err;
+    E->pinned_step = &E->pinned->step;
+    E->pinned_ctl = &E->pinned->ctl;
+    E->run_out = &E->pinned->run;
     int rc = setup_systems(E, why);
     if (rc) return bail(rc == -2 ? RDGPU_ERR_NOMEM : RDGPU_ERR_ARG, why);
     // the harmonic-repulsion-only fast path applies when every pair potential is
@@ -2107,10 +2250,13 @@ int create_impl(const rdgpu_system_desc* desc, int nsys, const rdgpu_box* boxes,
     // cells of all systems, for the cell walk
     rc = configure_cells(E, std::max(desc->cell_size, E->max_rc), why);
     if (rc) return bail(rc, why);
-    if (cudaMalloc(&E->ctl, sizeof(ListCtl)) != cudaSuccess ||
-        cudaMallocHost(&E->pinned_ctl, sizeof(ListCtl)) != cudaSuccess)
+    // the list's control words and, after them, list_run_kernel's
+    constexpr size_t run_at = 256;
+    static_assert(sizeof(ListCtl) <= run_at, "control words overlap");
+    if (cudaMalloc(&E->ctl, run_at + 2 * sizeof(RunCtl)) != cudaSuccess)
         return bail(RDGPU_ERR_NOMEM, "device allocation failed");
-    cudaMemsetAsync(E->ctl, 0, sizeof(ListCtl), E->stream);
+    E->run_ctl = (RunCtl*)((char*)E->ctl + run_at);
+    cudaMemsetAsync(E->ctl, 0, run_at + 2 * sizeof(RunCtl), E->stream);
     if (cudaStreamSynchronize(E->stream) != cudaSuccess) return bail(RDGPU_ERR_CUDA, "initialisation failed");
     if (E->nb_req == RDGPU_NB_LIST) {
         // a requested pair list that the boxes cannot hold falls back to the cell walk
@@ -2149,11 +2295,10 @@ int rdgpu_destroy(rdgpu_handle h)
     free_particles(E);
     dfree(E->sys_d); dfree(E->tab_d); dfree(E->ext_d); dfree(E->start); dfree(E->counts); dfree(E->tile_sum);
     dfree(E->err); dfree(E->err_step); dfree(E->step_d); dfree(E->ctl); dfree(E->rl2_d);
-    if (E->pinned_ctl) cudaFreeHost(E->pinned_ctl);
     dfree(E->red_d); dfree(E->redc_d); dfree(E->part_d); dfree(E->pcnt_d); dfree(E->ed_buf); dfree(E->off_d); dfree(E->rdf_acc); dfree(E->rdf_tmp); dfree(E->rdf_e2);
     dfree(E->rdf_grid_d); dfree(E->rdf_cnt); dfree(E->rdf_start); dfree(E->rdf_tsum); dfree(E->rdf_rec);
-    if (E->pinned_err) cudaFreeHost(E->pinned_err);
-    if (E->pinned_step) cudaFreeHost(E->pinned_step);
+    if (E->pinned) cudaFreeHost(E->pinned);
+    dfree(E->run_tsum);
     if (E->stream) cudaStreamDestroy(E->stream);
     if (E->stream2) cudaStreamDestroy(E->stream2);
     delete E;

@@ -108,16 +108,27 @@ template <> struct Acc<double> {
 // ---------------------------------------------------------------------------
 // state access
 // ---------------------------------------------------------------------------
+// Reads of data that a kernel of one step only reads go through the
+// non-coherent path (ldg).  COH: the same read as a plain load, for the
+// kernel of many steps (list_run_kernel), which writes those arrays itself
+// and orders the reads after the writes with its grid barrier.
+template <bool COH, class T> __device__ __forceinline__ T ld(const T* p)
+{
+    if constexpr (COH) return *p;
+    else return __ldg(p);
+}
+template <bool COH = false>
 __device__ __forceinline__ void load_pos(const State<float>& s, long long i, float x[3], int& w)
 {
-    const float4 p = __ldg(s.pos + i);
+    const float4 p = ld<COH>(s.pos + i);
     x[0] = p.x; x[1] = p.y; x[2] = p.z;
     w = __float_as_int(p.w);
 }
+template <bool COH = false>
 __device__ __forceinline__ void load_pos(const State<double>& s, long long i, double x[3], int& w)
 {
     const double2* p = reinterpret_cast<const double2*>(s.rec + i);
-    const double2 a = __ldg(p), b = __ldg(p + 1);
+    const double2 a = ld<COH>(p), b = ld<COH>(p + 1);
     x[0] = a.x; x[1] = a.y; x[2] = b.x;
     w = __double2loint(b.y);
 }
@@ -537,7 +548,7 @@ __device__ __forceinline__ int em_update(double x[3], double* /*c*/, int& w, con
 // forces (and, for MODE 1, half energies) of the bonds of particle id: one
 // pair potential each, at any distance, minimum image (the groups of
 // ReaDDy; CudaSimulation.cu:1829-1836 with each particle's own type)
-template <class R, int MODE>
+template <class R, int MODE, bool COH = false>
 __device__ __forceinline__ void bond_forces(const Args<R>& a, const State<R>& st, int id, const R xi[3],
                                             const SysDev& s, Acc<R>& acc)
 {
@@ -547,7 +558,7 @@ __device__ __forceinline__ void bond_forces(const Args<R>& a, const State<R>& st
         const int j = a.inv[a.bpart[b]];
         R xj[3];
         int wj;
-        load_pos(st, j, xj, wj);
+        load_pos<COH>(st, j, xj, wj);
         const R dx = mimg_sel(xi[0], xj[0], bx.L[0], bx.half[0], s.per[0]);
         const R dy = mimg_sel(xi[1], xj[1], bx.L[1], bx.half[1], s.per[1]);
         const R dz = mimg_sel(xi[2], xj[2], bx.L[2], bx.half[2], s.per[2]);
@@ -1910,72 +1921,70 @@ __device__ __forceinline__ void quad_entries(const int4& q, int k0, int i, int* 
     }
 }
 
-// one BD step of every particle over its pair list; ALLPER: every axis of
-// every system is periodic (the minimum image needs no per-axis test);
-// NARROW: list entries are 16-bit offsets (the handle's list format).  The
-// FP32 harmonic-repulsion kernel of all-periodic systems runs 9 blocks of 128
-// per SM (56 registers, no spill), measured 4 % faster than 8; 10 spill, and
-// so do the other FP32 variants at 9.  Its FP64 twin runs 7 (72 registers,
-// 3 % faster than 6 despite a few spilled registers; 8 is slower).
-template <class R, bool HREP, bool ALLPER, int BLOCK, bool NARROW>
-__global__ void __launch_bounds__(BLOCK, (sizeof(R) == 4 ? (HREP && ALLPER ? 1152 : 1024) : (HREP && ALLPER ? 896 : 768)) /
-                                             BLOCK)
-    list_step_kernel(Args<R> a, ListArgs<R> v)
-{
-    __shared__ R s_rc2[MAXT * MAXT];
-    __shared__ FastTab<R> s_ft;
-    // the error flag, the step counter and the buffer parity, then the
-    // particle's inputs, all requested before the pair tables: the block
-    // waits on one round of loads, not three
-    const int err0 = *((volatile int*)a.err);
-    const long long t = *((volatile const long long*)a.step_ptr) + a.step_off;
-    const int nreb = *((volatile const int*)&v.ctl->nreb);
-    const int sel = (int)((t + (long long)nreb) & 1LL);
-    const State<R> cur = sel ? v.b1 : v.b0;
-    const State<R> nxt = sel ? v.b0 : v.b1;
-    if (err0) return;   // an earlier step failed: keep its input intact
-    const int i = blockIdx.x * BLOCK + threadIdx.x;
-    const bool live = i < a.ntot;
-    int si = 0;
-    R xi[3] = {R(0), R(0), R(0)};
-    int wi = 0;
-    R c[3] = {R(0), R(0), R(0)};
-    int id = 0;
-    uint2 hd = make_uint2(0, 0);
-    int4 q0 = make_int4(0, 0, 0, 0), q1 = q0;
-    if (live) {
+// what the list step reads of particle i before its partners: state, list
+// head and the first 8 list entries (one narrow group, two wide ones; the
+// capacity is >= 8), before the list length is known; entries past it are
+// unused
+template <class R, bool NARROW, bool COH> struct ListIn {
+    int si, wi, id;
+    R xi[3], c[3];
+    uint2 hd;
+    int4 q0, q1;
+    __device__ __forceinline__ void clear()
+    {
+        si = wi = id = 0;
+        xi[0] = xi[1] = xi[2] = R(0);
+        c[0] = c[1] = c[2] = R(0);
+        hd = make_uint2(0, 0);
+        q0 = q1 = make_int4(0, 0, 0, 0);
+    }
+    __device__ __forceinline__ void load(const Args<R>& a, const ListArgs<R>& v, const State<R>& cur, int i)
+    {
         si = a.sys_of[i];
-        load_pos(cur, i, xi, wi);
+        load_pos<COH>(cur, i, xi, wi);
         if constexpr (sizeof(R) == 4) {
-            const float4 q = __ldg(cur.aux + i);
+            const float4 q = ld<COH>(cur.aux + i);
             c[0] = q.x; c[1] = q.y; c[2] = q.z;
             id = __float_as_int(q.w);
         } else {
-            id = __ldg(&cur.rec[i].id);
+            id = ld<COH>(&cur.rec[i].id);
         }
-        hd = __ldg(v.head + i);
-        // the first 8 list entries (one narrow group, two wide ones; capacity
-        // >= 8), before the list length is known; entries past it are unused
-        q0 = __ldg(v.nbr + i);
-        q1 = NARROW ? q0 : __ldg(v.nbr + i + v.stride);
+        hd = ld<COH>(v.head + i);
+        q0 = ld<COH>(v.nbr + i);
+        q1 = NARROW ? q0 : ld<COH>(v.nbr + i + v.stride);
     }
-    // rows of the S types in use (entries (ti, tj) with ti >= S are never read)
-    for (int k = threadIdx.x; k < MAXT * a.tab->S; k += BLOCK) {
-        s_rc2[k] = a.tab->rc2[k];
+};
+
+// the pair tables of a block: rows of the S types in use (entries (ti, tj)
+// with ti >= S are never read)
+template <class R, bool HREP>
+__device__ __forceinline__ void load_pair_tables(const TypeTab<R>* tab, R* s_rc2, FastTab<R>& s_ft)
+{
+    for (int k = threadIdx.x; k < MAXT * tab->S; k += blockDim.x) {
+        s_rc2[k] = tab->rc2[k];
         if (HREP) {
-            s_ft.k[k] = a.tab->nterm[k] ? a.tab->term[k * MAX_TERMS].k : R(0);
-            s_ft.r0[k] = a.tab->nterm[k] ? a.tab->term[k * MAX_TERMS].r0 : R(0);
+            s_ft.k[k] = tab->nterm[k] ? tab->term[k * MAX_TERMS].k : R(0);
+            s_ft.r0[k] = tab->nterm[k] ? tab->term[k * MAX_TERMS].r0 : R(0);
         }
     }
-    __syncthreads();
-    if (!live) return;
-    const SysDev& s = a.sys[si];
-    const int ti = wi & 0xff;
+}
+
+// One BD step (number t) of particle i over its pair list: the new state to
+// nxt; returns the error flags and, in dd, the squared displacement since
+// the build (lattice estimate; the thresholds allow for its error).
+template <class R, bool HREP, bool ALLPER, bool NARROW, bool COH>
+__device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>& v, const State<R>& cur,
+                                             const State<R>& nxt, int i, ListIn<R, NARROW, COH>& in, long long t,
+                                             const R* __restrict__ s_rc2, const FastTab<R>& s_ft, float& dd)
+{
+    R* xi = in.xi;
+    const SysDev& s = a.sys[in.si];
+    const int ti = in.wi & 0xff;
     Box<R> bx;
     bx.load(s);
     Acc<R> acc;
     acc.zero();
-    const int cnt = head_count(hd);
+    const int cnt = head_count(in.hd);
     const int4* nb4 = v.nbr + i;
     PairFrame pf;
     double il[3] = {0.0, 0.0, 0.0};
@@ -1997,9 +2006,9 @@ __global__ void __launch_bounds__(BLOCK, (sizeof(R) == 4 ? (HREP && ALLPER ? 115
             const int kq = (k0 & ~3) + 4 * h;       // the quad's first entry
             const int gi = kq / EPG;                // and its group
             int4 q = make_int4(0, 0, 0, 0);
-            if (gi == 0) q = q0;
-            else if (gi == 1 && !NARROW) q = q1;
-            else if (kq < cnt) q = __ldg(nb4 + (long long)gi * v.stride);
+            if (gi == 0) q = in.q0;
+            else if (gi == 1 && !NARROW) q = in.q1;
+            else if (kq < cnt) q = ld<COH>(nb4 + (long long)gi * v.stride);
             quad_entries<NARROW>(q, kq, i, jj + 4 * h);
         }
         if (LCHUNK == 2 && (k0 & 2)) { jj[0] = jj[2]; jj[1] = jj[3]; }   // the quad's upper pair
@@ -2017,7 +2026,7 @@ __global__ void __launch_bounds__(BLOCK, (sizeof(R) == 4 ? (HREP && ALLPER ? 115
         int wj[LCHUNK];
 #pragma unroll
         for (int u = 0; u < LCHUNK; ++u) {
-            if (HREP || jj[u] >= 0) load_pos(cur, jj[u], xj[u], wj[u]);
+            if (HREP || jj[u] >= 0) load_pos<COH>(cur, jj[u], xj[u], wj[u]);
             else { xj[u][0] = xj[u][1] = xj[u][2] = R(0); wj[u] = 0; }
         }
 #pragma unroll
@@ -2054,39 +2063,82 @@ __global__ void __launch_bounds__(BLOCK, (sizeof(R) == 4 ? (HREP && ALLPER ? 115
             }
         }
     }
-    if (a.bstart) bond_forces<R, 0>(a, cur, id, xi, s, acc);
+    if (a.bstart) bond_forces<R, 0, COH>(a, cur, in.id, xi, s, acc);
     R F[3];
     acc.force(F);
     if (a.n_ext > 0) {
-        const ExtTerm<R>* ep = a.ext + (long long)si * a.n_ext;
+        const ExtTerm<R>* ep = a.ext + (long long)in.si * a.n_ext;
         R ee = R(0);
         for (int e = 0; e < a.n_ext; ++e)
             if ((ep[e].tmask >> ti) & 1u) ext_force(ep[e], a.tab->prad[ti], xi, F, ee);
     }
     R xn[3];
     if (a.noise) {
-        const double* nz = a.noise + 3 * (s.part_base + id);
+        const double* nz = a.noise + 3 * (s.part_base + in.id);
         xn[0] = (R)nz[0]; xn[1] = (R)nz[1]; xn[2] = (R)nz[2];
     } else {
-        bd_normals(s.seed, t, (long long)id, xn);
+        bd_normals(s.seed, t, (long long)in.id, xn);
     }
-    const int ef = em_update<ALLPER>(xi, c, wi, F, xn, a.tab->a[ti], a.tab->b[ti], s);
-    // displacement since the build (lattice estimate; the thresholds
-    // allow for its error)
-    const float dd = head_disp2(hd, xi, s);
-    if (dd > v.cap2) *((volatile int*)&v.ctl->need) = 1;
-    const bool hot = dd > v.thr2;
+    const int ef = em_update<ALLPER>(xi, in.c, in.wi, F, xn, a.tab->a[ti], a.tab->b[ti], s);
+    dd = head_disp2(in.hd, xi, s);
+    store_state(nxt, i, xi, in.wi, in.c, in.id);
+    return ef;
+}
+
+// collects the hot particles of a step (squared displacement dd above thr2)
+// and raises the rebuild flag beyond cap2
+__device__ __forceinline__ void list_collect_hot(float dd, float thr2, float cap2, int i, int* nhot, int* need,
+                                                 int* hot_list, int hot_max)
+{
+    if (dd > cap2) *((volatile int*)need) = 1;
+    const bool hot = dd > thr2;
     const unsigned act = __activemask();
     const unsigned hm = __ballot_sync(act, hot);
     if (hm) {
         const int lane = threadIdx.x & 31;
         const int lead = __ffs(hm) - 1;
         int base = 0;
-        if (lane == lead) base = atomicAdd(&v.ctl->nhot, __popc(hm));
+        if (lane == lead) base = atomicAdd(nhot, __popc(hm));
         base = __shfl_sync(act, base, lead) + __popc(hm & ((1u << lane) - 1u));
-        if (hot && base < v.hot_max) v.hot[base] = i;
+        if (hot && base < hot_max) hot_list[base] = i;
     }
-    store_state(nxt, i, xi, wi, c, id);
+}
+
+// one BD step of every particle over its pair list; ALLPER: every axis of
+// every system is periodic (the minimum image needs no per-axis test);
+// NARROW: list entries are 16-bit offsets (the handle's list format).  The
+// FP32 harmonic-repulsion kernel of all-periodic systems runs 9 blocks of 128
+// per SM (56 registers, no spill), measured 4 % faster than 8; 10 spill, and
+// so do the other FP32 variants at 9.  Its FP64 twin runs 7 (72 registers,
+// 3 % faster than 6 despite a few spilled registers; 8 is slower).
+template <class R, bool HREP, bool ALLPER, int BLOCK, bool NARROW>
+__global__ void __launch_bounds__(BLOCK, (sizeof(R) == 4 ? (HREP && ALLPER ? 1152 : 1024) : (HREP && ALLPER ? 896 : 768)) /
+                                             BLOCK)
+    list_step_kernel(Args<R> a, ListArgs<R> v)
+{
+    __shared__ R s_rc2[MAXT * MAXT];
+    __shared__ FastTab<R> s_ft;
+    // the error flag, the step counter and the buffer parity, then the
+    // particle's inputs, all requested before the pair tables: the block
+    // waits on one round of loads, not three
+    const int err0 = *((volatile int*)a.err);
+    const long long t = *((volatile const long long*)a.step_ptr) + a.step_off;
+    const int nreb = *((volatile const int*)&v.ctl->nreb);
+    const int sel = (int)((t + (long long)nreb) & 1LL);
+    const State<R> cur = sel ? v.b1 : v.b0;
+    const State<R> nxt = sel ? v.b0 : v.b1;
+    if (err0) return;   // an earlier step failed: keep its input intact
+    const int i = blockIdx.x * BLOCK + threadIdx.x;
+    const bool live = i < a.ntot;
+    ListIn<R, NARROW, false> in;
+    in.clear();
+    if (live) in.load(a, v, cur, i);
+    load_pair_tables<R, HREP>(a.tab, s_rc2, s_ft);
+    __syncthreads();
+    if (!live) return;
+    float dd;
+    const int ef = list_step_one<R, HREP, ALLPER, NARROW, false>(a, v, cur, nxt, i, in, t, s_rc2, s_ft, dd);
+    list_collect_hot(dd, v.thr2, v.cap2, i, &v.ctl->nhot, &v.ctl->need, v.hot, v.hot_max);
     if (ef) {
         atomicOr(a.err, ef);
         atomicMin((unsigned long long*)a.err_step, (unsigned long long)t);
@@ -2158,14 +2210,14 @@ struct ListWriter {
 };
 
 // appends the pairs of one candidate range closer than their list radius
-template <class R>
+template <class R, bool COH>
 __device__ __forceinline__ void list_range(const State<R>& st, int j0, int j1, int self, const R xi[3], R sx, R sy,
                                            R sz, const R* __restrict__ rl2, ListWriter& lw, int& cnt)
 {
     for (int j = j0; j < j1; ++j) {
         R xj[3];
         int wj;
-        load_pos(st, j, xj, wj);
+        load_pos<COH>(st, j, xj, wj);
         const R dx = sub_rn(xi[0], add_rn(xj[0], sx));
         const R dy = sub_rn(xi[1], add_rn(xj[1], sy));
         const R dz = sub_rn(xi[2], add_rn(xj[2], sz));
@@ -2242,15 +2294,16 @@ __device__ __forceinline__ void list_row_ranges(const Args<R>& a, const SysDev& 
     f(a.start[row + xa], a.start[row + xb + 1], R(0), sy, sz);
 }
 
-// the pair list of sorted particle i from its 27-cell neighbourhood
-template <class R>
-__device__ __forceinline__ void list_build_one(const Args<R>& a, const ListArgs<R>& v, const State<R>& st, int i,
-                                               const R* __restrict__ s_rl2, long long off)
+// the pair list of sorted particle i from its 27-cell neighbourhood; returns
+// EF_LISTOVF / EF_LISTWIDE when it does not fit, cnt its length
+template <class R, bool COH>
+__device__ __forceinline__ int list_build_one(const Args<R>& a, const ListArgs<R>& v, const State<R>& st, int i,
+                                              const R* __restrict__ s_rl2, int& cnt)
 {
     const SysDev& s = a.sys[a.sys_of[i]];
     R xi[3];
     int wi;
-    load_pos(st, i, xi, wi);
+    load_pos<COH>(st, i, xi, wi);
     const R* rl2 = s_rl2 + (wi & 0xff) * MAXT;
     ListWriter lw;
     lw.nbr = v.nbr;
@@ -2259,14 +2312,14 @@ __device__ __forceinline__ void list_build_one(const Args<R>& a, const ListArgs<
     lw.cap = v.cap;
     lw.narrow = v.narrow != 0;
     lw.wide_need = false;
-    int cnt = 0;
+    cnt = 0;
     ListCell<R> g;
     g.locate(s, xi);
     const R lim = v.rl2max * R(1.0001);
     for (int dz = -1; dz <= 1; ++dz)
         for (int dy = -1; dy <= 1; ++dy)
             list_row_ranges<R>(a, s, g, lim, dz, dy, [&](int j0, int j1, R sx, R sy, R sz) {
-                list_range<R>(st, j0, j1, i, xi, sx, sy, sz, rl2, lw, cnt);
+                list_range<R, COH>(st, j0, j1, i, xi, sx, sy, sz, rl2, lw, cnt);
             });
     // narrow lists: the rest of the last group (all of group 0 for an empty
     // list: the list step always loads it) holds offset 0, the particle
@@ -2276,11 +2329,7 @@ __device__ __forceinline__ void list_build_one(const Args<R>& a, const ListArgs<
         for (int k = cnt; k < kfill; ++k) lw.put(k, i);
     }
     v.head[i] = make_head(xi, s, min(cnt, v.cap));
-    if (cnt > v.cap || lw.wide_need) {
-        if (cnt > v.cap) atomicMax(&v.ctl->maxcnt, cnt);
-        atomicOr(a.err, (cnt > v.cap ? EF_LISTOVF : 0) | (lw.wide_need ? EF_LISTWIDE : 0));
-        atomicMin((unsigned long long*)a.err_step, (unsigned long long)(*a.step_ptr + off));
-    }
+    return (cnt > v.cap ? EF_LISTOVF : 0) | (lw.wide_need ? EF_LISTWIDE : 0);
 }
 
 // re-sort, part 4: the pair list of every particle of the re-sorted state.
@@ -2299,18 +2348,25 @@ __global__ void __launch_bounds__(BLOCK) list_build_kernel(Args<R> a, ListArgs<R
     const int sel = list_sel(a, v, off);
     const State<R> st = sel ? v.b0 : v.b1;     // the scatter's destination
     const int i = blockIdx.x * BLOCK + threadIdx.x;
-    if (i < a.ntot) list_build_one<R>(a, v, st, i, s_rl2, off);
+    if (i >= a.ntot) return;
+    int cnt;
+    const int ef = list_build_one<R, false>(a, v, st, i, s_rl2, cnt);
+    if (ef) {
+        if (ef & EF_LISTOVF) atomicMax(&v.ctl->maxcnt, cnt);
+        atomicOr(a.err, ef);
+        atomicMin((unsigned long long*)a.err_step, (unsigned long long)(*a.step_ptr + off));
+    }
 }
 
 // j is in the pair list of i
-template <class R>
+template <class R, bool COH>
 __device__ __forceinline__ bool listed(const ListArgs<R>& v, int i, int j)
 {
-    const int cnt = head_count(__ldg(v.head + i));
+    const int cnt = head_count(ld<COH>(v.head + i));
     const int4* nb4 = v.nbr + i;
     const int epg = v.narrow ? 8 : 4;
     for (int k0 = 0; k0 < cnt; k0 += epg) {
-        const int4 q = __ldg(nb4 + (long long)(k0 / epg) * v.stride);
+        const int4 q = ld<COH>(nb4 + (long long)(k0 / epg) * v.stride);
         for (int u = 0; u < epg && k0 + u < cnt; ++u)
             if (list_entry(q, u, v.narrow != 0, i) == j) return true;
     }
@@ -2320,14 +2376,14 @@ __device__ __forceinline__ bool listed(const ListArgs<R>& v, int i, int j)
 // every particle now closer to hot particle h than their cutoff is in h's
 // list, and h in its; one warp per hot particle, lane r < 9 walks cell row r
 // of the 27-cell neighbourhood
-template <class R>
+template <class R, bool COH = false>
 __device__ __forceinline__ bool hot_pairs_listed(const Args<R>& a, const ListArgs<R>& v, const State<R>& st, int h,
                                                  int lane)
 {
     const SysDev& s = a.sys[a.sys_of[h]];
     R xh[3];
     int wh;
-    load_pos(st, h, xh, wh);
+    load_pos<COH>(st, h, xh, wh);
     bool ok = true;
     if (lane < 9) {
         const R* rc2 = a.tab->rc2 + (wh & 0xff) * MAXT;
@@ -2342,7 +2398,7 @@ __device__ __forceinline__ bool hot_pairs_listed(const Args<R>& a, const ListArg
                 R xj[4][3];
                 int wj[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) load_pos(st, min(j + u, j1 - 1), xj[u], wj[u]);
+                for (int u = 0; u < 4; ++u) load_pos<COH>(st, min(j + u, j1 - 1), xj[u], wj[u]);
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const int jj = j + u;
@@ -2350,7 +2406,7 @@ __device__ __forceinline__ bool hot_pairs_listed(const Args<R>& a, const ListArg
                     const R dx = mimg_sel(xh[0], xj[u][0], bx.L[0], bx.half[0], s.per[0]);
                     const R dy = mimg_sel(xh[1], xj[u][1], bx.L[1], bx.half[1], s.per[1]);
                     const R dz = mimg_sel(xh[2], xj[u][2], bx.L[2], bx.half[2], s.per[2]);
-                    if (dist2(dx, dy, dz) < rc2[wj[u] & 0xff] * R(1.0001) && !(listed(v, h, jj) && listed(v, jj, h)))
+                    if (dist2(dx, dy, dz) < rc2[wj[u] & 0xff] * R(1.0001) && !(listed<R, COH>(v, h, jj) && listed<R, COH>(v, jj, h)))
                         ok = false;
                 }
             }

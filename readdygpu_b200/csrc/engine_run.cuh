@@ -1,0 +1,404 @@
+// engine_run.cuh -- the pair-list steps of one rdgpu_step call in one launch.
+//
+// list_run_kernel advances a handle by up to nsteps steps: a cooperative grid
+// (all blocks resident) steps every particle, meets at a grid barrier, and
+// goes on with the next step; the list check of a step runs together with the
+// next step, and the re-sort and list build run inside the same kernel when
+// they are due.  Launched step by step (list_step_kernel, list_check_kernel
+// and a conditional graph node per step), 8 to 40 us of every step went to
+// launch gaps, the check's own launch and the conditional node: more than the
+// step itself up to about a million particles.  Per step, launch by launch
+// and in one launch (tuned, steps of a 100-step frame): 1,000 particles FP64
+// 19.7 and 10.0 us, 20,000 FP64 22.2 and 11.6, 250,000 (vesicle, FP32C) 56.7
+// and 47.1, 370,000 FP64 in 64 systems 54.5 and 38.0, 2.9 M in 512 systems
+// 158 and 152 (there the step and the list build are bound by issue).
+#pragma once
+#include "engine_kernels.cuh"
+
+namespace rdgpu {
+
+// Control words of one launch, zero at its start.  A launch zeroes the next
+// one's (two of them alternate), so no memset is queued per call.
+struct RunCtl {
+    unsigned bar;                             // blocks that arrived at grid barriers so far
+    int dead;                                 // a barrier wait ran out
+    int nhot[3], need[3], fail[3], err[3];    // per step attempt, used in turn
+    int lerr, maxcnt;                         // list build: EF_LIST*, longest list
+};
+
+// The launch's outcome, written to page-locked host memory by its last act.
+struct RunOut {
+    int err;        // EF_*: of step t (its input is intact), or of the build for step t's input
+    int dead;       // a barrier wait ran out: the state is undefined
+    int sel;        // the buffer that holds the input of step t
+    int builds;     // list builds in this launch
+    int maxcnt;     // longest list met by an overflowing build
+    int pad;
+    long long t;    // the next step to compute
+};
+
+template <class R> struct RunArgs {
+    Args<R> a;
+    ListArgs<R> v;
+    RunCtl* ctl;
+    RunCtl* next;      // the next launch's, zeroed by this one
+    RunOut* out;
+    int* tile_sum;     // one per scan tile (run_scan_tile cells each)
+    long long ncells;
+    long long t0;      // first step
+    int nsteps;
+    int sel0;          // the buffer that holds its input
+};
+
+// Threads per block and blocks per SM, at most: the occupancy of the step
+// kernel of the same variant (list_step_kernel), in few, large blocks, so
+// that few arrive at the grid barrier.
+template <class R, bool HREP, bool ALLPER> struct RunShape {
+    static constexpr bool FAST = HREP && ALLPER;
+    static constexpr int BLOCK = sizeof(R) == 4 ? (FAST ? 384 : 512) : (FAST ? 448 : 384);
+    static constexpr int PER_SM = sizeof(R) == 4 && FAST ? 3 : 2;
+};
+
+// a wait at the grid barrier gives up after this many polls (some seconds)
+constexpr unsigned RUN_POLLS = 1u << 23;
+
+constexpr int RUN_SCAN_PER = 8;       // cells per thread and scan tile
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
+{
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// block-wide words of list_run_kernel
+struct RunShared {
+    int flags[5];     // dead, nhot, need, fail, err of the slot read at the last barrier
+    int lerr;
+    int next;         // next work item of the block
+    int warp[32];     // block scan
+    unsigned bars;    // grid barriers passed
+};
+
+// Grid barrier: everything written before it by any block is visible after it
+// to plain loads of every block (release by the arriving thread after the
+// block's barrier, acquire before the block's second one).  The flags of
+// attempt slot `slot` come with it, and the block's work counter restarts.
+// False when the wait ran out (every block then leaves the kernel).
+__device__ __forceinline__ bool run_sync(RunCtl* c, RunShared& sh, int slot)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&c->bar, 1u);
+        const unsigned target = (sh.bars += 1u) * gridDim.x;
+        unsigned polls = 0;
+        while (ld_acquire(&c->bar) < target && ++polls < RUN_POLLS) {}
+        if (polls >= RUN_POLLS) atomicExch(&c->dead, 1);
+        __threadfence();
+        volatile const RunCtl* v = c;
+        sh.flags[0] = v->dead;
+        sh.flags[1] = v->nhot[slot];
+        sh.flags[2] = v->need[slot];
+        sh.flags[3] = v->fail[slot];
+        sh.flags[4] = v->err[slot];
+        sh.lerr = v->lerr;
+        sh.next = blockDim.x >> 5;
+    }
+    __syncthreads();
+    return sh.flags[0] == 0;
+}
+
+// next work item of the calling warp within its block
+__device__ __forceinline__ int run_next(RunShared& sh)
+{
+    int w = 0;
+    if ((threadIdx.x & 31) == 0) w = atomicAdd(&sh.next, 1);
+    return __shfl_sync(FULL, w, 0);
+}
+
+// The block's q-th tile of 32 particles: single tiles dealt to the blocks in
+// turn, and drawn from the block's counter by its warps, so that systems of
+// different density spread over all blocks (runs of 8 tiles, for partners
+// shared in L1, measured 2 to 4 % slower from 250,000 particles up: the blocks
+// then end apart by up to a fifth of a step).
+__device__ __forceinline__ int run_tile(int q) { return q * (int)gridDim.x + (int)blockIdx.x; }
+
+// Cell starts from the counts (cleared on the way), as scan_tiles_kernel and
+// scan_apply_kernel do in two launches: tile sums, a grid barrier, then each
+// tile's exclusive prefix.  A tile is RUN_SCAN_PER cells per thread.
+__device__ __forceinline__ bool run_scan(RunCtl* c, RunShared& sh, int* counts, int* start, int* tile_sum,
+                                         long long ncells, int slot)
+{
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+    const long long per_tile = (long long)blockDim.x * RUN_SCAN_PER;
+    const int ntiles = (int)((ncells + per_tile - 1) / per_tile);
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const long long base = tile * per_tile + tid;
+        int sum = 0;
+#pragma unroll
+        for (int k = 0; k < RUN_SCAN_PER; ++k) {
+            const long long q = base + (long long)k * blockDim.x;
+            if (q < ncells) sum += counts[q];
+        }
+        sum = __reduce_add_sync(FULL, sum);
+        if (lane == 0) sh.warp[wid] = sum;
+        __syncthreads();
+        if (tid == 0) {
+            int tot = 0;
+            for (int w = 0; w < nw; ++w) tot += sh.warp[w];
+            tile_sum[tile] = tot;
+        }
+        __syncthreads();
+    }
+    if (!run_sync(c, sh, slot)) return false;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        int before = 0;
+        for (int k = tid; k < tile; k += blockDim.x) before += tile_sum[k];
+        // each thread scans RUN_SCAN_PER consecutive cells (32 bytes: whole sectors)
+        const long long q0 = tile * per_tile + (long long)tid * RUN_SCAN_PER;
+        alignas(16) int v[RUN_SCAN_PER];
+        int sum = 0;
+        const bool whole = q0 + RUN_SCAN_PER <= ncells;
+        if (whole) {
+            int4* c4 = reinterpret_cast<int4*>(counts + q0);
+            reinterpret_cast<int4*>(v)[0] = c4[0];
+            reinterpret_cast<int4*>(v)[1] = c4[1];
+            c4[0] = c4[1] = make_int4(0, 0, 0, 0);
+        } else {
+#pragma unroll
+            for (int k = 0; k < RUN_SCAN_PER; ++k) {
+                v[k] = 0;
+                if (q0 + k < ncells) {
+                    v[k] = counts[q0 + k];
+                    counts[q0 + k] = 0;
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < RUN_SCAN_PER; ++k) sum += v[k];
+        const int incl = warp_incl_scan(sum, lane);
+        before = __reduce_add_sync(FULL, before);
+        if (lane == 31) sh.warp[wid] = incl + before;     // the tiles before, as the warps found them
+        __syncthreads();
+        // base of this warp: all tiles before (every warp's share) and the
+        // warps before it in this tile
+        const int mine = __shfl_sync(FULL, incl, 31);
+        int all = 0;
+        for (int w = 0; w < nw; ++w) {
+            const int x = sh.warp[w];
+            all += x;
+        }
+        __syncthreads();
+        if (lane == 0) sh.warp[wid] = mine;
+        __syncthreads();
+        int inside = 0, upto = 0;
+        for (int w = 0; w < nw; ++w) {
+            const int x = sh.warp[w];
+            inside += x;
+            if (w < wid) upto += x;
+        }
+        int run = (all - inside) + upto + incl - sum;
+        alignas(16) int o[RUN_SCAN_PER];
+#pragma unroll
+        for (int k = 0; k < RUN_SCAN_PER; ++k) {
+            o[k] = run;
+            run += v[k];
+            if (q0 + k == ncells - 1) start[ncells] = run;
+        }
+        if (whole) {
+            reinterpret_cast<int4*>(start + q0)[0] = reinterpret_cast<int4*>(o)[0];
+            reinterpret_cast<int4*>(start + q0)[1] = reinterpret_cast<int4*>(o)[1];
+        } else {
+#pragma unroll
+            for (int k = 0; k < RUN_SCAN_PER; ++k)
+                if (q0 + k < ncells) start[q0 + k] = o[k];
+        }
+        __syncthreads();
+    }
+    return true;
+}
+
+// Re-sort by cell from src into dst and list build (list_count_kernel ..
+// list_build_kernel in one go).  False: a barrier wait ran out.  An
+// overflowing build leaves its flags in sh.lerr (the state in src is intact).
+template <class R>
+__device__ __noinline__ bool run_rebuild(const RunArgs<R>& p, RunShared& sh, R* s_rl2, int sel, int slot)
+{
+    const Args<R>& a = p.a;
+    const State<R> src = sel ? p.v.b1 : p.v.b0;
+    const State<R> dst = sel ? p.v.b0 : p.v.b1;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    for (long long i = first; i < a.ntot; i += stride) {
+        const SysDev& s = a.sys[a.sys_of[i]];
+        R x[3];
+        int w;
+        load_pos<true>(src, i, x, w);
+        int c[3];
+        cell_coords(s, x, c);
+        const long long cell = s.cell_base + ((long long)c[2] * s.n[1] + c[1]) * s.n[0] + c[0];
+        a.tslot[i] = atomicAdd(a.counts + cell, 1);
+        a.tcell[i] = (int)cell;
+    }
+    for (int k = threadIdx.x; k < MAXT * MAXT; k += blockDim.x) s_rl2[k] = p.v.rl2t[k];
+    if (!run_sync(p.ctl, sh, slot)) return false;
+    if (!run_scan(p.ctl, sh, a.counts, const_cast<int*>(a.start), p.tile_sum, p.ncells, slot)) return false;
+    if (!run_sync(p.ctl, sh, slot)) return false;
+    for (long long i = first; i < a.ntot; i += stride) {
+        const long long d = a.start[a.tcell[i]] + a.tslot[i];
+        if constexpr (sizeof(R) == 4) {
+            const float4 q = src.aux[i];
+            dst.pos[d] = src.pos[i];
+            dst.aux[d] = q;
+            if (a.inv) a.inv[__float_as_int(q.w)] = (int)d;
+        } else {
+            const Rec64 r = src.rec[i];
+            dst.rec[d] = r;
+            if (a.inv) a.inv[r.id] = (int)d;
+        }
+    }
+    if (!run_sync(p.ctl, sh, slot)) return false;
+    const int lane = threadIdx.x & 31;
+    const int tiles = (int)((a.ntot + 31) / 32);
+    for (int q = threadIdx.x >> 5;; q = run_next(sh)) {
+        const int tile = run_tile(q);
+        if (tile >= tiles) break;
+        const long long i = (long long)tile * 32 + lane;
+        if (i < a.ntot) {
+            int cnt;
+            const int ef = list_build_one<R, true>(a, p.v, dst, (int)i, s_rl2, cnt);
+            if (ef) {
+                if (ef & EF_LISTOVF) atomicMax(&p.ctl->maxcnt, cnt);
+                atomicOr(&p.ctl->lerr, ef);
+            }
+        }
+        __syncwarp();
+    }
+    return run_sync(p.ctl, sh, slot);
+}
+
+// Up to nsteps pair-list steps.  Step attempt n of the launch reads buffer
+// sel and writes the other one; its flags are in slot n % 3 and its hot
+// particles in half n & 1 of the hot list.  While it runs, warps check the
+// hot particles of the step before it (the state in buffer sel) against the
+// lists (list_check_kernel's test).  At the barrier that ends it every block
+// takes the same decision:
+//   - a pair was missing from the lists: attempt n is void (its input is
+//     intact), the input is re-sorted, the lists are built and the step is
+//     repeated;
+//   - an error: the launch ends with that step's input intact;
+//   - else the step stands; if it moved a particle too far (or made too many
+//     hot) its result is re-sorted and the lists are built.
+// So a step takes one grid barrier, and a pair that the lists miss costs a
+// repeated step (about one in 20 to 50).  The forces a repeated step sees are
+// those of a step after a separate check: the trajectory does not change.
+template <class R, bool HREP, bool ALLPER, bool NARROW>
+__global__ void __launch_bounds__(RunShape<R, HREP, ALLPER>::BLOCK, RunShape<R, HREP, ALLPER>::PER_SM)
+    list_run_kernel(const __grid_constant__ RunArgs<R> p)
+{
+    __shared__ R s_rc2[MAXT * MAXT];
+    __shared__ R s_rl2[MAXT * MAXT];
+    __shared__ FastTab<R> s_ft;
+    __shared__ RunShared sh;
+    const Args<R>& a = p.a;
+    const ListArgs<R>& v = p.v;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int G = gridDim.x, bid = blockIdx.x;
+    const int tiles = (int)((a.ntot + 31) / 32);
+    if (bid == 0 && threadIdx.x < sizeof(RunCtl) / sizeof(int)) reinterpret_cast<int*>(p.next)[threadIdx.x] = 0;
+    if (threadIdx.x == 0) {
+        sh.bars = 0;
+        sh.lerr = 0;
+        sh.next = blockDim.x >> 5;
+    }
+    load_pair_tables<R, HREP>(a.tab, s_rc2, s_ft);
+    __syncthreads();
+    long long t = p.t0;
+    int sel = p.sel0, n = 0, slot = 0, builds = 0, nhot = 0, err = 0;
+    bool alive = true;
+    const long long tend = p.t0 + p.nsteps;
+    while (t < tend) {
+        const State<R> cur = sel ? v.b1 : v.b0;
+        const State<R> nxt = sel ? v.b0 : v.b1;
+        const int after = slot == 2 ? 0 : slot + 1;
+        if (bid == 0 && threadIdx.x == 0) {
+            p.ctl->nhot[after] = 0;
+            p.ctl->need[after] = 0;
+            p.ctl->fail[after] = 0;
+            p.ctl->err[after] = 0;
+        }
+        const int* hot_in = v.hot + ((n & 1) ^ 1) * v.hot_max;
+        int* hot_out = v.hot + (n & 1) * v.hot_max;
+        // work items of this block: its share of the hot particles to check,
+        // then its tiles
+        const int hb = nhot > bid ? (nhot - bid + G - 1) / G : 0;
+        for (int w = warp;; w = run_next(sh)) {
+            if (w < hb) {
+                if (!hot_pairs_listed<R, true>(a, v, cur, hot_in[w * G + bid], lane) && lane == 0)
+                    *((volatile int*)&p.ctl->fail[slot]) = 1;
+                continue;
+            }
+            const int tile = run_tile(w - hb);
+            if (tile >= tiles) break;
+            const int i = tile * 32 + lane;
+            if (i < a.ntot) {
+                ListIn<R, NARROW, true> in;
+                in.load(a, v, cur, i);
+                float dd;
+                const int ef = list_step_one<R, HREP, ALLPER, NARROW, true>(a, v, cur, nxt, i, in, t, s_rc2, s_ft, dd);
+                list_collect_hot(dd, v.thr2, v.cap2, i, &p.ctl->nhot[slot], &p.ctl->need[slot], hot_out, v.hot_max);
+                if (ef) atomicOr(&p.ctl->err[slot], ef);
+            }
+            __syncwarp();
+        }
+        alive = run_sync(p.ctl, sh, slot);
+        if (!alive) break;
+        const int found = sh.flags[1], need = sh.flags[2], fail = sh.flags[3];
+        err = sh.flags[4];
+        ++n;
+        slot = after;
+        nhot = 0;
+        bool rebuild = fail != 0;
+        if (fail) {
+            err = 0;
+        } else {
+            if (err) break;
+            ++t;
+            sel ^= 1;
+            rebuild = need || found > v.hot_max;
+            if (!rebuild) nhot = found;
+        }
+        if (!rebuild && t == tend && nhot > 0) {
+            // the last step's hot particles
+            hot_in = v.hot + ((n & 1) ^ 1) * v.hot_max;
+            const State<R> last = sel ? v.b1 : v.b0;
+            for (int h = warp * G + bid; h < nhot; h += G * (int)(blockDim.x >> 5))
+                if (!hot_pairs_listed<R, true>(a, v, last, hot_in[h], lane) && lane == 0)
+                    *((volatile int*)&p.ctl->fail[slot]) = 1;
+            alive = run_sync(p.ctl, sh, slot);
+            if (!alive) break;
+            rebuild = sh.flags[3] != 0;
+        }
+        if (rebuild) {
+            nhot = 0;
+            alive = run_rebuild<R>(p, sh, s_rl2, sel, slot);
+            if (!alive) break;
+            err = sh.lerr;
+            if (err) break;
+            sel ^= 1;
+            ++builds;
+        }
+    }
+    if (bid == 0 && threadIdx.x == 0) {
+        volatile RunOut* o = p.out;
+        o->err = err;
+        o->dead = alive ? 0 : 1;
+        o->sel = sel;
+        o->builds = builds;
+        o->maxcnt = *((volatile int*)&p.ctl->maxcnt);
+        o->t = t;
+    }
+}
+
+}  // namespace rdgpu

@@ -1,0 +1,133 @@
+"""The pair-list steps of an AUTO handle run in one launch per rdgpu_step call
+(list_run_kernel): the trajectory is the cell walk's, bit for bit in FP32C and
+to rounding in FP64, at the sizes where its shape changes (32-particle tiles,
+4 tiles per block, one block per SM, several blocks per SM), for every
+potential path, across rebuilds and whatever the split of the steps."""
+import numpy as np
+import pytest
+
+from readdygpu_b200 import RdgpuError, _abi as A, configs
+from readdygpu_b200.system import System, ParticleType, PairPotential
+
+from .test_gpu_pairlist import cluster_system, same
+from .test_gpu_parity import Engine, small_config2
+
+pytestmark = pytest.mark.gpu
+
+
+def plain(n, per=(1, 1, 1)):
+    L = float(np.float32(max(40.0, 50.0 * (n / 1000.0) ** (1.0 / 3.0))))
+    sys_ = System([ParticleType("A", 1e6, 1.5), ParticleType("B", 5e5, 2.0)],
+                  pair=[PairPotential(A.P2_HARMONIC, [(0, 0), (0, 1), (1, 1)], 10.0, "repulsive")],
+                  kT=2.437, dt=1e-9, lo=(0, 0, 0), hi=(L, L, L), periodic=per)
+    xyz = np.random.default_rng(n).uniform(0.2 * L, 0.8 * L, (n, 3)) if 0 in per else \
+        np.random.default_rng(n).uniform(0, L, (n, 3))
+    return sys_, xyz, (np.arange(n) % 2).astype(np.int32)
+
+
+def both(prec, sys_, xyz, types, split, boxes=None, offsets=None):
+    """Final positions of the cell walk and of the run kernel, whose calls are one launch each."""
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision=prec, seed=3, boxes=boxes, neighbour_mode=mode) as e:
+            e.set_particles(xyz, types, offsets=offsets)
+            e.autotune()
+            m0 = e.metrics()
+            l0 = e.launch_count()
+            for n in split:
+                e.step(n)
+            if mode == "auto":
+                assert m0["neighbour_mode"] == "list"
+                assert e.launch_count() - l0 == len(split)
+            m = e.metrics()
+            assert m["step"] == sum(split)
+            out.append(e.get_particles()[0])
+    return out[0], out[1], m["list_builds"] - m0["list_builds"]
+
+
+# tiles of 32; blocks of 4 tiles on 148 SMs up to 18,944; one block per SM up
+# to 56,832 (FP32C) or 66,304 (FP64)
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+@pytest.mark.parametrize("n", [1, 33, 127, 1000, 18_945, 56_833, 66_305])
+def test_run_equals_cells_over_sizes(prec, n):
+    sys_, xyz, types = plain(n)
+    xc, xr, _ = both(prec, sys_, xyz, types, [1, 60, 39])
+    same(prec, xc, xr)
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+def test_run_equals_cells_over_rebuilds(prec):
+    """1,500 steps in one call (two launches), with many rebuilds inside them."""
+    sys_, xyz, types = plain(3000)
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision=prec, seed=3, neighbour_mode=mode) as e:
+            e.set_particles(xyz, types)
+            e.autotune()
+            b0 = e.metrics()["list_builds"]
+            e.step(1500)
+            m = e.metrics()
+            out.append(e.get_particles()[0])
+    assert m["neighbour_mode"] == "list" and m["list_builds"] - b0 > 10
+    same(prec, out[0], out[1])
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+def test_run_general_potentials_and_open_axes(prec):
+    """Weak attraction, a disk and an open z axis (the term-table variant)."""
+    sys_, xyz, types = small_config2(1000)
+    xc, xr, _ = both(prec, sys_, xyz, types, [130])
+    same(prec, xc, xr)
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+def test_run_open_axis_repulsion(prec):
+    """Harmonic repulsion with an open axis (the per-axis variant)."""
+    sys_, xyz, types = plain(2000, per=(1, 1, 0))
+    xc, xr, _ = both(prec, sys_, xyz, types, [130])
+    same(prec, xc, xr)
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+def test_run_batch_of_many_tiles(prec):
+    """An uneven batch of more tiles than warps on the GPU (runs of 8 tiles)."""
+    w = configs.config4(n_systems=140)
+    xc, xr, nb = both(prec, w.system, w.xyz, w.types, [100], boxes=w.boxes, offsets=w.offsets)
+    assert w.n > 32 * 4 * 148 * 36 and nb > 1
+    same(prec, xc, xr)
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+def test_run_overflow_regrows(prec):
+    """A cluster drawn together by attraction overflows the lists inside a call."""
+    sys_, xyz, types = cluster_system(n_gas=3000, n_cluster=60)
+    sys_.pair.append(PairPotential(A.P2_WEAK_PIECEWISE, [(0, 0)], 60.0, r0=2.0, length=4.0, depth=40.0))
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision=prec, seed=5, neighbour_mode=mode) as e:
+            e.set_particles(xyz, types)
+            e.autotune()
+            e.step(100)
+            out.append(e.get_particles()[0])
+    same(prec, out[0], out[1])
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+def test_run_reports_a_failed_step(prec):
+    """Two overlapping particles under an enormous force constant leave the box
+    by more than an edge in one step: the step is reported and its input stays,
+    as with the cell walk."""
+    res = []
+    for mode in ("cells", "auto"):
+        sys_, xyz, types = plain(500)
+        sys_.pair[0].k = 1e12
+        xyz[1] = xyz[0] + 0.3
+        with Engine(sys_, precision=prec, seed=5, neighbour_mode=mode) as e:
+            e.set_particles(xyz, types)
+            with pytest.raises(RdgpuError) as err:
+                e.autotune()
+                e.step(50)
+            res.append((err.value.code, str(err.value).split("at step")[-1]))
+            x, _ = e.get_particles()
+            assert np.isfinite(x).all()
+    assert res[0] == res[1]
