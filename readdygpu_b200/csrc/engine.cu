@@ -1043,7 +1043,8 @@ template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E
         grid = (int)std::min<long long>((long long)sms * S::PER_SM, (tiles + wpb - 1) / wpb);
     }
     void* args[] = {&p};
-    CK(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(block), args, 0, E->stream));
+    CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_dyn_bytes<R>(S::BLOCK)));
+    CK(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(block), args, run_dyn_bytes<R>(block), E->stream));
     ++E->launches;
     return RDGPU_OK;
 }

@@ -64,6 +64,10 @@ constexpr unsigned RUN_POLLS = 1u << 23;
 
 constexpr int RUN_SCAN_PER = 8;       // cells per thread and scan tile
 
+// dynamic shared memory: the squared list radii, then list_build_one's scratch
+extern __shared__ __align__(16) char run_dyn[];
+template <class R> constexpr size_t run_dyn_bytes(int block) { return MAXT * MAXT * sizeof(R) + (size_t)block * LB_BYTES; }
+
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
 {
     unsigned v;
@@ -223,8 +227,10 @@ __device__ __forceinline__ bool run_scan(RunCtl* c, RunShared& sh, int* counts, 
 // list_build_kernel in one go).  False: a barrier wait ran out.  An
 // overflowing build leaves its flags in sh.lerr (the state in src is intact).
 template <class R>
-__device__ __noinline__ bool run_rebuild(const RunArgs<R>& p, RunShared& sh, R* s_rl2, int sel, int slot)
+__device__ __noinline__ bool run_rebuild(const RunArgs<R>& p, RunShared& sh, int sel, int slot)
 {
+    R* s_rl2 = reinterpret_cast<R*>(run_dyn);
+    char* scratch = run_dyn + MAXT * MAXT * sizeof(R);
     const Args<R>& a = p.a;
     const State<R> src = sel ? p.v.b1 : p.v.b0;
     const State<R> dst = sel ? p.v.b0 : p.v.b1;
@@ -267,7 +273,7 @@ __device__ __noinline__ bool run_rebuild(const RunArgs<R>& p, RunShared& sh, R* 
         const long long i = (long long)tile * 32 + lane;
         if (i < a.ntot) {
             int cnt;
-            const int ef = list_build_one<R, true>(a, p.v, dst, (int)i, s_rl2, cnt);
+            const int ef = list_build_one<R, true>(a, p.v, dst, (int)i, s_rl2, scratch, cnt);
             if (ef) {
                 if (ef & EF_LISTOVF) atomicMax(&p.ctl->maxcnt, cnt);
                 atomicOr(&p.ctl->lerr, ef);
@@ -298,7 +304,6 @@ __global__ void __launch_bounds__(RunShape<R, HREP, ALLPER>::BLOCK, RunShape<R, 
     list_run_kernel(const __grid_constant__ RunArgs<R> p)
 {
     __shared__ R s_rc2[MAXT * MAXT];
-    __shared__ R s_rl2[MAXT * MAXT];
     __shared__ FastTab<R> s_ft;
     __shared__ RunShared sh;
     const Args<R>& a = p.a;
@@ -382,7 +387,7 @@ __global__ void __launch_bounds__(RunShape<R, HREP, ALLPER>::BLOCK, RunShape<R, 
         }
         if (rebuild) {
             nhot = 0;
-            alive = run_rebuild<R>(p, sh, s_rl2, sel, slot);
+            alive = run_rebuild<R>(p, sh, sel, slot);
             if (!alive) break;
             err = sh.lerr;
             if (err) break;
