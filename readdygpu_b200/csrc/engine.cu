@@ -1020,9 +1020,9 @@ template <class R> int capture_list_graph(Engine* E, int n, cudaGraphExec_t* out
 
 // list_run_kernel with as many threads per particle tile as the GPU has room
 // for: up to 4 tiles per SM, one block of 4 warps on as many SMs as it takes
-// (the fewer warps an SM runs, the sooner each is done); up to a block per
-// SM, all SMs with the warps their tiles need; beyond that, all blocks that
-// fit.  Blocks of 128 or 256 threads on the same number of warps measured 15
+// (the fewer warps an SM runs, the sooner each is done); beyond that, as many
+// blocks on every SM, with as many warps each, as the tiles need and the SM
+// holds.  Blocks of 128 or 256 threads on the same number of warps measured 15
 // to 35 % slower at 250,000 particles (more arrivals at the barrier, shares
 // that differ more).
 template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E, RunArgs<R>& p)
@@ -1035,12 +1035,11 @@ template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E
     if (tiles <= 4LL * sms) {
         block = 128;
         grid = (int)((tiles + 3) / 4);
-    } else if (tiles <= (long long)sms * (S::BLOCK / 32)) {
-        block = 32 * (int)((tiles + sms - 1) / sms);
-        grid = sms;
     } else {
-        constexpr int wpb = S::BLOCK / 32;
-        grid = (int)std::min<long long>((long long)sms * S::PER_SM, (tiles + wpb - 1) / wpb);
+        int per = 1;
+        while (per < S::PER_SM && tiles > (long long)sms * per * (S::BLOCK / 32)) ++per;
+        grid = sms * per;
+        block = 32 * (int)std::min<long long>(S::BLOCK / 32, (tiles + grid - 1) / grid);
     }
     void* args[] = {&p};
     CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_dyn_bytes<R>(S::BLOCK)));

@@ -1955,17 +1955,18 @@ template <class R, bool NARROW, bool COH> struct ListIn {
     }
 };
 
-// the pair tables of a block: rows of the S types in use (entries (ti, tj)
-// with ti >= S are never read)
+// The pair tables of a block: rows of the S types in use (entries (ti, tj)
+// with ti >= S are never read).  one[]: the pair has at most one term, a
+// harmonic repulsion (k, r0 in the FastTab; with HREP every pair has).
 template <class R, bool HREP>
-__device__ __forceinline__ void load_pair_tables(const TypeTab<R>* tab, R* s_rc2, FastTab<R>& s_ft)
+__device__ __forceinline__ void load_pair_tables(const TypeTab<R>* tab, R* s_rc2, FastTab<R>& s_ft, bool* s_one)
 {
     for (int k = threadIdx.x; k < MAXT * tab->S; k += blockDim.x) {
         s_rc2[k] = tab->rc2[k];
-        if (HREP) {
-            s_ft.k[k] = tab->nterm[k] ? tab->term[k * MAX_TERMS].k : R(0);
-            s_ft.r0[k] = tab->nterm[k] ? tab->term[k * MAX_TERMS].r0 : R(0);
-        }
+        const PairTerm<R>& t = tab->term[k * MAX_TERMS];
+        s_ft.k[k] = tab->nterm[k] ? t.k : R(0);
+        s_ft.r0[k] = tab->nterm[k] ? t.r0 : R(0);
+        if (!HREP) s_one[k] = tab->nterm[k] <= 1 && t.kind == 1 && t.sub == 2;
     }
 }
 
@@ -1975,7 +1976,8 @@ __device__ __forceinline__ void load_pair_tables(const TypeTab<R>* tab, R* s_rc2
 template <class R, bool HREP, bool ALLPER, bool NARROW, bool COH>
 __device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>& v, const State<R>& cur,
                                              const State<R>& nxt, int i, ListIn<R, NARROW, COH>& in, long long t,
-                                             const R* __restrict__ s_rc2, const FastTab<R>& s_ft, float& dd)
+                                             const R* __restrict__ s_rc2, const FastTab<R>& s_ft,
+                                             const bool* __restrict__ s_one, float& dd)
 {
     R* xi = in.xi;
     const SysDev& s = a.sys[in.si];
@@ -1995,10 +1997,10 @@ __device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>
     constexpr int EPG = NARROW ? 8 : 4;      // entries per group
     constexpr int LCHUNK = sizeof(R) == 4 ? LIST_CHUNK : LIST_CHUNK_F64;
     static_assert(LCHUNK == 2 || LCHUNK % 4 == 0, "pairs or whole quads per chunk");
-    // FP32 HREP: every lane runs the warp's longest list (its chunks past its
-    // own list hold only itself), so the loop needs no per-lane exit (1 %
-    // faster on config 4; the FP64 step measured 2 % slower with it)
-    const int kend = (HREP && sizeof(R) == 4) ? __reduce_max_sync(__activemask(), cnt) : cnt;
+    // FP32: every lane runs the warp's longest list (its chunks past its own
+    // list hold only itself), so the loop needs no per-lane exit (1 % faster
+    // on config 4; the FP64 step measured 2 % slower with it)
+    const int kend = sizeof(R) == 4 ? __reduce_max_sync(__activemask(), cnt) : cnt;
     for (int k0 = 0; k0 < kend; k0 += LCHUNK) {
         int jj[LCHUNK < 4 ? 4 : LCHUNK];
 #pragma unroll
@@ -2012,26 +2014,22 @@ __device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>
             quad_entries<NARROW>(q, kq, i, jj + 4 * h);
         }
         if (LCHUNK == 2 && (k0 & 2)) { jj[0] = jj[2]; jj[1] = jj[3]; }   // the quad's upper pair
-        // entries past the list's end: HREP, the particle itself (r^2 = 0,
-        // no force, and its position is in L1), which spares the chunk's
-        // per-entry branches; otherwise -1 (skipped).  Narrow lists hold
-        // offset 0 (the particle itself) in the rest of their last group, and
-        // a group past the list's end is not loaded (zeros, offset 0 again),
-        // so HREP needs no test there
-        if constexpr (!(HREP && NARROW)) {
+        // Entries past the list's end are the particle itself (r^2 = 0, no
+        // force, and its position is in L1), which spares the chunk's
+        // per-entry branches.  Narrow lists hold offset 0 (the particle
+        // itself) in the rest of their last group, and a group past the
+        // list's end is not loaded (zeros, offset 0 again), so they need no
+        // test.
+        if constexpr (!NARROW) {
 #pragma unroll
-            for (int u = 0; u < LCHUNK; ++u) jj[u] = (k0 + u < cnt) ? jj[u] : (HREP ? i : -1);
+            for (int u = 0; u < LCHUNK; ++u) jj[u] = (k0 + u < cnt) ? jj[u] : i;
         }
         R xj[LCHUNK][3];
         int wj[LCHUNK];
 #pragma unroll
-        for (int u = 0; u < LCHUNK; ++u) {
-            if (HREP || jj[u] >= 0) load_pos<COH>(cur, jj[u], xj[u], wj[u]);
-            else { xj[u][0] = xj[u][1] = xj[u][2] = R(0); wj[u] = 0; }
-        }
+        for (int u = 0; u < LCHUNK; ++u) load_pos<COH>(cur, jj[u], xj[u], wj[u]);
 #pragma unroll
         for (int u = 0; u < LCHUNK; ++u) {
-            if (!HREP && jj[u] < 0) continue;
             R dx, dy, dz, r2;
             if constexpr (sizeof(R) == 4) {
                 pair_disp_x2(pf, xj[u][0], xj[u][1], xj[u][2], dx, dy, dz, r2);
@@ -2051,13 +2049,20 @@ __device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>
                         else { const R r = sqrt(r2); pre = s_ft.k[pidx] * (r - s_ft.r0[pidx]) / r; }
                         acc.add(pre, dx, dy, dz);
                     }
-                } else {
+                } else if (r2 > R(0)) {
+                    // (a coincident pair has no direction: every term times
+                    // a zero displacement)
                     const R r = sqrt(r2);
-                    const int nt = a.tab->nterm[pidx];
-                    for (int m = 0; m < nt; ++m) {
-                        R pre, e;
-                        pair_term(a.tab->term[pidx * MAX_TERMS + m], r, pre, e);
-                        acc.add(pre, dx, dy, dz);
+                    if (s_one[pidx]) {
+                        const R r0 = s_ft.r0[pidx];
+                        if (r < r0) acc.add(s_ft.k[pidx] * (r - r0) / r, dx, dy, dz);
+                    } else {
+                        const int nt = a.tab->nterm[pidx];
+                        for (int m = 0; m < nt; ++m) {
+                            R pre, e;
+                            pair_term(a.tab->term[pidx * MAX_TERMS + m], r, pre, e);
+                            acc.add(pre, dx, dy, dz);
+                        }
                     }
                 }
             }
@@ -2118,6 +2123,7 @@ __global__ void __launch_bounds__(BLOCK, (sizeof(R) == 4 ? (HREP && ALLPER ? 115
 {
     __shared__ R s_rc2[MAXT * MAXT];
     __shared__ FastTab<R> s_ft;
+    __shared__ bool s_one[HREP ? 1 : MAXT * MAXT];
     // the error flag, the step counter and the buffer parity, then the
     // particle's inputs, all requested before the pair tables: the block
     // waits on one round of loads, not three
@@ -2133,11 +2139,11 @@ __global__ void __launch_bounds__(BLOCK, (sizeof(R) == 4 ? (HREP && ALLPER ? 115
     ListIn<R, NARROW, false> in;
     in.clear();
     if (live) in.load(a, v, cur, i);
-    load_pair_tables<R, HREP>(a.tab, s_rc2, s_ft);
+    load_pair_tables<R, HREP>(a.tab, s_rc2, s_ft, s_one);
     __syncthreads();
     if (!live) return;
     float dd;
-    const int ef = list_step_one<R, HREP, ALLPER, NARROW, false>(a, v, cur, nxt, i, in, t, s_rc2, s_ft, dd);
+    const int ef = list_step_one<R, HREP, ALLPER, NARROW, false>(a, v, cur, nxt, i, in, t, s_rc2, s_ft, s_one, dd);
     list_collect_hot(dd, v.thr2, v.cap2, i, &v.ctl->nhot, &v.ctl->need, v.hot, v.hot_max);
     if (ef) {
         atomicOr(a.err, ef);

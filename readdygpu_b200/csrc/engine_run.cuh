@@ -305,6 +305,7 @@ __global__ void __launch_bounds__(RunShape<R, HREP, ALLPER>::BLOCK, RunShape<R, 
 {
     __shared__ R s_rc2[MAXT * MAXT];
     __shared__ FastTab<R> s_ft;
+    __shared__ bool s_one[HREP ? 1 : MAXT * MAXT];
     __shared__ RunShared sh;
     const Args<R>& a = p.a;
     const ListArgs<R>& v = p.v;
@@ -317,7 +318,7 @@ __global__ void __launch_bounds__(RunShape<R, HREP, ALLPER>::BLOCK, RunShape<R, 
         sh.lerr = 0;
         sh.next = blockDim.x >> 5;
     }
-    load_pair_tables<R, HREP>(a.tab, s_rc2, s_ft);
+    load_pair_tables<R, HREP>(a.tab, s_rc2, s_ft, s_one);
     __syncthreads();
     long long t = p.t0;
     int sel = p.sel0, n = 0, slot = 0, builds = 0, nhot = 0, err = 0;
@@ -351,7 +352,8 @@ __global__ void __launch_bounds__(RunShape<R, HREP, ALLPER>::BLOCK, RunShape<R, 
                 ListIn<R, NARROW, true> in;
                 in.load(a, v, cur, i);
                 float dd;
-                const int ef = list_step_one<R, HREP, ALLPER, NARROW, true>(a, v, cur, nxt, i, in, t, s_rc2, s_ft, dd);
+                const int ef = list_step_one<R, HREP, ALLPER, NARROW, true>(a, v, cur, nxt, i, in, t, s_rc2, s_ft,
+                                                                               s_one, dd);
                 list_collect_hot(dd, v.thr2, v.cap2, i, &p.ctl->nhot[slot], &p.ctl->need[slot], hot_out, v.hot_max);
                 if (ef) atomicOr(&p.ctl->err[slot], ef);
             }
