@@ -1018,29 +1018,18 @@ template <class R> int capture_list_graph(Engine* E, int n, cudaGraphExec_t* out
     return RDGPU_OK;
 }
 
-// list_run_kernel with as many threads per particle tile as the GPU has room
-// for: up to 4 tiles per SM, one block of 4 warps on as many SMs as it takes
-// (the fewer warps an SM runs, the sooner each is done); beyond that, as many
-// blocks on every SM, with as many warps each, as the tiles need and the SM
-// holds.  Blocks of 128 or 256 threads on the same number of warps measured 15
-// to 35 % slower at 250,000 particles (more arrivals at the barrier, shares
-// that differ more).
+// list_run_kernel with one block per SM: up to 4 tiles of 32 particles per SM,
+// blocks of 4 warps on as many SMs as it takes (the fewer warps an SM runs, the
+// sooner each is done); beyond that a warp per tile on every SM, up to the
+// block's limit.
 template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E, RunArgs<R>& p)
 {
     using S = RunShape<R, HREP, ALLPER>;
     const void* f = (const void*)list_run_kernel<R, HREP, ALLPER, NARROW>;
     const long long tiles = (E->npart_tot + 31) / 32;
     const int sms = E->sm_count;
-    int block = S::BLOCK, grid = 1;
-    if (tiles <= 4LL * sms) {
-        block = 128;
-        grid = (int)((tiles + 3) / 4);
-    } else {
-        int per = 1;
-        while (per < S::PER_SM && tiles > (long long)sms * per * (S::BLOCK / 32)) ++per;
-        grid = sms * per;
-        block = 32 * (int)std::min<long long>(S::BLOCK / 32, (tiles + grid - 1) / grid);
-    }
+    const int block = tiles <= 4LL * sms ? 128 : 32 * (int)std::min<long long>(S::BLOCK / 32, (tiles + sms - 1) / sms);
+    const int grid = tiles <= 4LL * sms ? (int)((tiles + 3) / 4) : sms;
     void* args[] = {&p};
     CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_dyn_bytes<R>(S::BLOCK)));
     CK(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(block), args, run_dyn_bytes<R>(block), E->stream));

@@ -50,13 +50,14 @@ template <class R> struct RunArgs {
     int sel0;          // the buffer that holds its input
 };
 
-// Threads per block and blocks per SM, at most: the occupancy of the step
-// kernel of the same variant (list_step_kernel), in few, large blocks, so
-// that few arrive at the grid barrier.
+// Threads per block, at most; one block per SM.  Its warps draw the SM's tiles
+// from one counter, and 148 blocks arrive at the grid barrier: against 3 blocks
+// of 384 (FP32C repulsion), 2 of 512 (FP32C) or 2 of 448 and 384 (FP64) 135 ->
+// 130 us a step on 2.9 M particles in 512 systems, 39.4 -> 35.1 us on 250,000
+// (vesicle), 36.0 -> 34.7 us on 370,000 FP64 in 64 systems and 25.9 -> 21.0 us
+// on 60,000 FP64 (vesicle).  64 registers a thread FP32, 72 and 80 FP64.
 template <class R, bool HREP, bool ALLPER> struct RunShape {
-    static constexpr bool FAST = HREP && ALLPER;
-    static constexpr int BLOCK = sizeof(R) == 4 ? (FAST ? 384 : 512) : (FAST ? 448 : 384);
-    static constexpr int PER_SM = sizeof(R) == 4 && FAST ? 3 : 2;
+    static constexpr int BLOCK = sizeof(R) == 4 ? 1024 : (HREP && ALLPER ? 896 : 768);
 };
 
 // a wait at the grid barrier gives up after this many polls (some seconds)
@@ -300,7 +301,7 @@ __device__ __noinline__ bool run_rebuild(const RunArgs<R>& p, RunShared& sh, int
 // repeated step (about one in 20 to 50).  The forces a repeated step sees are
 // those of a step after a separate check: the trajectory does not change.
 template <class R, bool HREP, bool ALLPER, bool NARROW>
-__global__ void __launch_bounds__(RunShape<R, HREP, ALLPER>::BLOCK, RunShape<R, HREP, ALLPER>::PER_SM)
+__global__ void __launch_bounds__(RunShape<R, HREP, ALLPER>::BLOCK, 1)
     list_run_kernel(const __grid_constant__ RunArgs<R> p)
 {
     __shared__ R s_rc2[MAXT * MAXT];

@@ -45,10 +45,10 @@ def both(prec, sys_, xyz, types, split, boxes=None, offsets=None):
     return out[0], out[1], m["list_builds"] - m0["list_builds"]
 
 
-# tiles of 32; blocks of 4 tiles on 148 SMs up to 18,944; one block per SM up
-# to 56,832 (FP32C) or 66,304 (FP64)
+# tiles of 32; blocks of 4 tiles on 148 SMs up to 18,944; a warp per tile up
+# to 151,552 (FP32C) or 132,608 (FP64)
 @pytest.mark.parametrize("prec", ["f32c", "f64"])
-@pytest.mark.parametrize("n", [1, 33, 127, 1000, 18_945, 56_833, 66_305])
+@pytest.mark.parametrize("n", [1, 33, 127, 1000, 18_945, 132_609, 151_553])
 def test_run_equals_cells_over_sizes(prec, n):
     sys_, xyz, types = plain(n)
     xc, xr, _ = both(prec, sys_, xyz, types, [1, 60, 39])
@@ -90,10 +90,10 @@ def test_run_open_axis_repulsion(prec):
 
 @pytest.mark.parametrize("prec", ["f32c", "f64"])
 def test_run_batch_of_many_tiles(prec):
-    """An uneven batch of more tiles than warps on the GPU (runs of 8 tiles)."""
+    """An uneven batch of several tiles per warp."""
     w = configs.config4(n_systems=140)
     xc, xr, nb = both(prec, w.system, w.xyz, w.types, [100], boxes=w.boxes, offsets=w.offsets)
-    assert w.n > 32 * 4 * 148 * 36 and nb > 1
+    assert w.n > 4 * 32 * 148 * 32 and nb > 1
     same(prec, xc, xr)
 
 
