@@ -1018,23 +1018,36 @@ template <class R> int capture_list_graph(Engine* E, int n, cudaGraphExec_t* out
     return RDGPU_OK;
 }
 
-// list_run_kernel with one block per SM: up to 4 tiles of 32 particles per SM,
-// blocks of 4 warps on as many SMs as it takes (the fewer warps an SM runs, the
-// sooner each is done); beyond that a warp per tile on every SM, up to the
-// block's limit.
-template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E, RunArgs<R>& p)
+template <class R> int launch_run_as(Engine* E, RunArgs<R>& p, const void* f, int block, int most, int grid)
 {
-    using S = RunShape<R, HREP, ALLPER>;
-    const void* f = (const void*)list_run_kernel<R, HREP, ALLPER, NARROW>;
-    const long long tiles = (E->npart_tot + 31) / 32;
-    const int sms = E->sm_count;
-    const int block = tiles <= 4LL * sms ? 128 : 32 * (int)std::min<long long>(S::BLOCK / 32, (tiles + sms - 1) / sms);
-    const int grid = tiles <= 4LL * sms ? (int)((tiles + 3) / 4) : sms;
     void* args[] = {&p};
-    CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_dyn_bytes<R>(S::BLOCK)));
+    CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_dyn_bytes<R>(most)));
     CK(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(block), args, run_dyn_bytes<R>(block), E->stream));
     ++E->launches;
     return RDGPU_OK;
+}
+
+// list_run_kernel with one block per SM: up to RUN_HOME_MANY tiles of 32
+// particles per SM, a warp per tile that keeps it and the rest of the block for
+// the hot particles (narrow lists); beyond that a warp per tile that an SM gets,
+// up to the block's limit.
+template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E, RunArgs<R>& p)
+{
+    const long long tiles = (E->npart_tot + 31) / 32;
+    const int sms = E->sm_count;
+    const int grid = (int)std::min<long long>(sms, tiles);
+    const long long per_sm = (tiles + grid - 1) / grid;
+    if constexpr (NARROW) {
+        if (per_sm <= RUN_HOME_FEW)
+            return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_HOME_FEW>,
+                                 32 * ((int)per_sm + 4), run_home_block(RUN_HOME_FEW), grid);
+        if (per_sm <= RUN_HOME_MANY)
+            return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_HOME_MANY>,
+                                 32 * ((int)per_sm + 3), run_home_block(RUN_HOME_MANY), grid);
+    }
+    constexpr int most = RunShape<R, HREP, ALLPER>::BLOCK;
+    const int block = 32 * (int)std::max<long long>(4, std::min<long long>(most / 32, per_sm));
+    return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, NARROW, 0>, block, most, grid);
 }
 
 template <class R, bool NARROW> int launch_run_w(Engine* E, RunArgs<R>& p, bool allper)

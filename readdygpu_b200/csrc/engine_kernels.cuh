@@ -1970,22 +1970,18 @@ __device__ __forceinline__ void load_pair_tables(const TypeTab<R>* tab, R* s_rc2
     }
 }
 
-// One BD step (number t) of particle i over its pair list: the new state to
-// nxt; returns the error flags and, in dd, the squared displacement since
-// the build (lattice estimate; the thresholds allow for its error).
-template <class R, bool HREP, bool ALLPER, bool NARROW, bool COH>
-__device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>& v, const State<R>& cur,
-                                             const State<R>& nxt, int i, ListIn<R, NARROW, COH>& in, long long t,
-                                             const R* __restrict__ s_rc2, const FastTab<R>& s_ft,
-                                             const bool* __restrict__ s_one, float& dd)
+// The pair forces on particle i over its list.  LCHUNK: entries whose positions
+// are requested together; SECOND: the second narrow group is in in.q1.
+template <class R, bool HREP, bool NARROW, bool COH, int LCHUNK, bool SECOND>
+__device__ __forceinline__ void list_pairs(const Args<R>& a, const ListArgs<R>& v, const State<R>& cur, int i,
+                                           const ListIn<R, NARROW, COH>& in, const SysDev& s,
+                                           const R* __restrict__ s_rc2, const FastTab<R>& s_ft,
+                                           const bool* __restrict__ s_one, Acc<R>& acc)
 {
-    R* xi = in.xi;
-    const SysDev& s = a.sys[in.si];
+    const R* xi = in.xi;
     const int ti = in.wi & 0xff;
     Box<R> bx;
     bx.load(s);
-    Acc<R> acc;
-    acc.zero();
     const int cnt = head_count(in.hd);
     const int4* nb4 = v.nbr + i;
     PairFrame pf;
@@ -1995,7 +1991,6 @@ __device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>
     // the partners in chunks of LCHUNK entries (4 or 8): all their positions
     // are requested before the first pair is evaluated
     constexpr int EPG = NARROW ? 8 : 4;      // entries per group
-    constexpr int LCHUNK = sizeof(R) == 4 ? LIST_CHUNK : LIST_CHUNK_F64;
     static_assert(LCHUNK == 2 || LCHUNK % 4 == 0, "pairs or whole quads per chunk");
     // FP32: every lane runs the warp's longest list (its chunks past its own
     // list hold only itself), so the loop needs no per-lane exit (1 % faster
@@ -2009,7 +2004,7 @@ __device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>
             const int gi = kq / EPG;                // and its group
             int4 q = make_int4(0, 0, 0, 0);
             if (gi == 0) q = in.q0;
-            else if (gi == 1 && !NARROW) q = in.q1;
+            else if (gi == 1 && (!NARROW || SECOND)) q = in.q1;
             else if (kq < cnt) q = ld<COH>(nb4 + (long long)gi * v.stride);
             quad_entries<NARROW>(q, kq, i, jj + 4 * h);
         }
@@ -2068,6 +2063,19 @@ __device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>
             }
         }
     }
+}
+
+// One BD step of particle i from its pair forces and the step's noise (drawn
+// by noise() last, when the fewest registers are held): the new state to in
+// and to nxt; returns the error flags and, in dd, the squared displacement
+// since the build (lattice estimate; the thresholds allow for its error).
+template <class R, bool ALLPER, bool NARROW, bool COH, class N>
+__device__ __forceinline__ int list_move(const Args<R>& a, const State<R>& cur, const State<R>& nxt, int i,
+                                         ListIn<R, NARROW, COH>& in, const SysDev& s, Acc<R>& acc, N&& noise,
+                                         float& dd)
+{
+    R* xi = in.xi;
+    const int ti = in.wi & 0xff;
     if (a.bstart) bond_forces<R, 0, COH>(a, cur, in.id, xi, s, acc);
     R F[3];
     acc.force(F);
@@ -2078,16 +2086,33 @@ __device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>
             if ((ep[e].tmask >> ti) & 1u) ext_force(ep[e], a.tab->prad[ti], xi, F, ee);
     }
     R xn[3];
-    if (a.noise) {
-        const double* nz = a.noise + 3 * (s.part_base + in.id);
-        xn[0] = (R)nz[0]; xn[1] = (R)nz[1]; xn[2] = (R)nz[2];
-    } else {
-        bd_normals(s.seed, t, (long long)in.id, xn);
-    }
+    noise(xn);
     const int ef = em_update<ALLPER>(xi, in.c, in.wi, F, xn, a.tab->a[ti], a.tab->b[ti], s);
     dd = head_disp2(in.hd, xi, s);
     store_state(nxt, i, xi, in.wi, in.c, in.id);
     return ef;
+}
+
+// One BD step (number t) of particle i over its pair list.
+template <class R, bool HREP, bool ALLPER, bool NARROW, bool COH>
+__device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>& v, const State<R>& cur,
+                                             const State<R>& nxt, int i, ListIn<R, NARROW, COH>& in, long long t,
+                                             const R* __restrict__ s_rc2, const FastTab<R>& s_ft,
+                                             const bool* __restrict__ s_one, float& dd)
+{
+    const SysDev& s = a.sys[in.si];
+    Acc<R> acc;
+    acc.zero();
+    list_pairs<R, HREP, NARROW, COH, sizeof(R) == 4 ? LIST_CHUNK : LIST_CHUNK_F64, false>(a, v, cur, i, in, s, s_rc2,
+                                                                                          s_ft, s_one, acc);
+    return list_move<R, ALLPER>(a, cur, nxt, i, in, s, acc, [&](R* xn) {
+        if (a.noise) {
+            const double* nz = a.noise + 3 * (s.part_base + in.id);
+            xn[0] = (R)nz[0]; xn[1] = (R)nz[1]; xn[2] = (R)nz[2];
+        } else {
+            bd_normals(s.seed, t, (long long)in.id, xn);
+        }
+    }, dd);
 }
 
 // collects the hot particles of a step (squared displacement dd above thr2)

@@ -60,6 +60,19 @@ template <class R, bool HREP, bool ALLPER> struct RunShape {
     static constexpr int BLOCK = sizeof(R) == 4 ? 1024 : (HREP && ALLPER ? 896 : 768);
 };
 
+// HOME > 0, for up to HOME tiles per SM (narrow lists): a warp keeps one tile
+// for the whole launch, its particles' state and first list groups in
+// registers, reads only partners from memory, and draws the next step's noise
+// while the barrier completes; 3 or 4 more warps check the hot particles.  Per
+// step, tiles read anew and kept: 1,000 particles FP64 9.8 and 7.3 us, FP32C
+// 7.6 and 6.0, 20,000 FP64 11.2 and 8.6, 30,000 FP32C 8.7 and 7.4, 60,000 FP64
+// (vesicle) 21.3 and 18.7 us.  Two sizes, 168 and 128 registers a thread: 13
+// for all costs the small ones 2 to 5 %; 22 (80 registers) is no gain.
+constexpr int RUN_HOME_FEW = 8;
+constexpr int RUN_HOME_MANY = 13;
+constexpr int run_home_block(int home) { return home == RUN_HOME_FEW ? 384 : 512; }
+template <class R> constexpr int RUN_HOME_CHUNK = sizeof(R) == 4 ? 8 : 4;   // partners requested together
+
 // a wait at the grid barrier gives up after this many polls (some seconds)
 constexpr unsigned RUN_POLLS = 1u << 23;
 
@@ -89,13 +102,19 @@ struct RunShared {
 // to plain loads of every block (release by the arriving thread after the
 // block's barrier, acquire before the block's second one).  The flags of
 // attempt slot `slot` come with it, and the block's work counter restarts.
-// False when the wait ran out (every block then leaves the kernel).
-__device__ __forceinline__ bool run_sync(RunCtl* c, RunShared& sh, int slot)
+// False when the wait ran out (every block then leaves the kernel).  Every
+// thread calls meanwhile() between the block's arrival and the wait.
+template <class F>
+__device__ __forceinline__ bool run_sync(RunCtl* c, RunShared& sh, int slot, F&& meanwhile)
 {
+    const bool leader = threadIdx.x == blockDim.x - 32;      // of the last warp (HOME: without a tile)
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (leader) {
         __threadfence();
         atomicAdd(&c->bar, 1u);
+    }
+    meanwhile();
+    if (leader) {
         const unsigned target = (sh.bars += 1u) * gridDim.x;
         unsigned polls = 0;
         while (ld_acquire(&c->bar) < target && ++polls < RUN_POLLS) {}
@@ -112,6 +131,11 @@ __device__ __forceinline__ bool run_sync(RunCtl* c, RunShared& sh, int slot)
     }
     __syncthreads();
     return sh.flags[0] == 0;
+}
+
+__device__ __forceinline__ bool run_sync(RunCtl* c, RunShared& sh, int slot)
+{
+    return run_sync(c, sh, slot, [] {});
 }
 
 // next work item of the calling warp within its block
@@ -300,8 +324,8 @@ __device__ __noinline__ bool run_rebuild(const RunArgs<R>& p, RunShared& sh, int
 // So a step takes one grid barrier, and a pair that the lists miss costs a
 // repeated step (about one in 20 to 50).  The forces a repeated step sees are
 // those of a step after a separate check: the trajectory does not change.
-template <class R, bool HREP, bool ALLPER, bool NARROW>
-__global__ void __launch_bounds__(RunShape<R, HREP, ALLPER>::BLOCK, 1)
+template <class R, bool HREP, bool ALLPER, bool NARROW, int HOME>
+__global__ void __launch_bounds__(HOME ? run_home_block(HOME) : RunShape<R, HREP, ALLPER>::BLOCK, 1)
     list_run_kernel(const __grid_constant__ RunArgs<R> p)
 {
     __shared__ R s_rc2[MAXT * MAXT];
@@ -325,6 +349,14 @@ __global__ void __launch_bounds__(RunShape<R, HREP, ALLPER>::BLOCK, 1)
     int sel = p.sel0, n = 0, slot = 0, builds = 0, nhot = 0, err = 0;
     bool alive = true;
     const long long tend = p.t0 + p.nsteps;
+    // HOME: this thread's particle
+    const int home_warps = (tiles + G - 1) / G;
+    const int hi = (warp * G + bid) * 32 + lane;
+    const bool home = HOME > 0 && warp < home_warps && hi < a.ntot;
+    bool loaded = false;
+    ListIn<R, NARROW, true> hin;
+    SysDev hs;
+    R hn[3];
     while (t < tend) {
         const State<R> cur = sel ? v.b1 : v.b0;
         const State<R> nxt = sel ? v.b0 : v.b1;
@@ -337,30 +369,59 @@ __global__ void __launch_bounds__(RunShape<R, HREP, ALLPER>::BLOCK, 1)
         }
         const int* hot_in = v.hot + ((n & 1) ^ 1) * v.hot_max;
         int* hot_out = v.hot + (n & 1) * v.hot_max;
-        // work items of this block: its share of the hot particles to check,
-        // then its tiles
-        const int hb = nhot > bid ? (nhot - bid + G - 1) / G : 0;
-        for (int w = warp;; w = run_next(sh)) {
-            if (w < hb) {
-                if (!hot_pairs_listed<R, true>(a, v, cur, hot_in[w * G + bid], lane) && lane == 0)
-                    *((volatile int*)&p.ctl->fail[slot]) = 1;
-                continue;
-            }
-            const int tile = run_tile(w - hb);
-            if (tile >= tiles) break;
-            const int i = tile * 32 + lane;
-            if (i < a.ntot) {
-                ListIn<R, NARROW, true> in;
-                in.load(a, v, cur, i);
+        if constexpr (HOME > 0) {
+            if (warp >= home_warps) {
+                const int spare = (int)(blockDim.x >> 5) - home_warps;
+                for (int h = (warp - home_warps) * G + bid; h < nhot; h += spare * G)
+                    if (!hot_pairs_listed<R, true>(a, v, cur, hot_in[h], lane) && lane == 0)
+                        *((volatile int*)&p.ctl->fail[slot]) = 1;
+            } else if (home) {
+                if (!loaded) {
+                    hin.load(a, v, cur, hi);
+                    hin.q1 = head_count(hin.hd) > 8 ? v.nbr[hi + v.stride] : make_int4(0, 0, 0, 0);
+                    hs = a.sys[hin.si];
+                    bd_normals(hs.seed, t, (long long)hin.id, hn);
+                }
+                Acc<R> acc;
+                acc.zero();
+                list_pairs<R, HREP, NARROW, true, RUN_HOME_CHUNK<R>, true>(a, v, cur, hi, hin, hs, s_rc2, s_ft,
+                                                                                          s_one, acc);
                 float dd;
-                const int ef = list_step_one<R, HREP, ALLPER, NARROW, true>(a, v, cur, nxt, i, in, t, s_rc2, s_ft,
-                                                                               s_one, dd);
-                list_collect_hot(dd, v.thr2, v.cap2, i, &p.ctl->nhot[slot], &p.ctl->need[slot], hot_out, v.hot_max);
+                const int ef = list_move<R, ALLPER>(a, cur, nxt, hi, hin, hs, acc, [&](R* xn) {
+                    xn[0] = hn[0]; xn[1] = hn[1]; xn[2] = hn[2];
+                }, dd);
+                list_collect_hot(dd, v.thr2, v.cap2, hi, &p.ctl->nhot[slot], &p.ctl->need[slot], hot_out, v.hot_max);
                 if (ef) atomicOr(&p.ctl->err[slot], ef);
             }
-            __syncwarp();
+            loaded = true;
+        } else {
+            // work items of this block: its share of the hot particles to check,
+            // then its tiles
+            const int hb = nhot > bid ? (nhot - bid + G - 1) / G : 0;
+            for (int w = warp;; w = run_next(sh)) {
+                if (w < hb) {
+                    if (!hot_pairs_listed<R, true>(a, v, cur, hot_in[w * G + bid], lane) && lane == 0)
+                        *((volatile int*)&p.ctl->fail[slot]) = 1;
+                    continue;
+                }
+                const int tile = run_tile(w - hb);
+                if (tile >= tiles) break;
+                const int i = tile * 32 + lane;
+                if (i < a.ntot) {
+                    ListIn<R, NARROW, true> in;
+                    in.load(a, v, cur, i);
+                    float dd;
+                    const int ef = list_step_one<R, HREP, ALLPER, NARROW, true>(a, v, cur, nxt, i, in, t, s_rc2, s_ft,
+                                                                                   s_one, dd);
+                    list_collect_hot(dd, v.thr2, v.cap2, i, &p.ctl->nhot[slot], &p.ctl->need[slot], hot_out, v.hot_max);
+                    if (ef) atomicOr(&p.ctl->err[slot], ef);
+                }
+                __syncwarp();
+            }
         }
-        alive = run_sync(p.ctl, sh, slot);
+        alive = run_sync(p.ctl, sh, slot, [&] {
+            if (HOME > 0 && home) bd_normals(hs.seed, t + 1, (long long)hin.id, hn);
+        });
         if (!alive) break;
         const int found = sh.flags[1], need = sh.flags[2], fail = sh.flags[3];
         err = sh.flags[4];
@@ -395,6 +456,7 @@ __global__ void __launch_bounds__(RunShape<R, HREP, ALLPER>::BLOCK, 1)
             err = sh.lerr;
             if (err) break;
             sel ^= 1;
+            loaded = false;
             ++builds;
         }
     }

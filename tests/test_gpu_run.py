@@ -45,10 +45,10 @@ def both(prec, sys_, xyz, types, split, boxes=None, offsets=None):
     return out[0], out[1], m["list_builds"] - m0["list_builds"]
 
 
-# tiles of 32; blocks of 4 tiles on 148 SMs up to 18,944; a warp per tile up
-# to 151,552 (FP32C) or 132,608 (FP64)
+# tiles of 32 particles on 148 SMs: warps that keep their tile up to 37,888 and
+# 61,568 particles (two block sizes), a warp per tile up to 132,608 (FP64) and 151,552 (FP32C)
 @pytest.mark.parametrize("prec", ["f32c", "f64"])
-@pytest.mark.parametrize("n", [1, 33, 127, 1000, 18_945, 132_609, 151_553])
+@pytest.mark.parametrize("n", [1, 33, 1000, 4737, 37_888, 37_889, 61_569, 132_609, 151_553])
 def test_run_equals_cells_over_sizes(prec, n):
     sys_, xyz, types = plain(n)
     xc, xr, _ = both(prec, sys_, xyz, types, [1, 60, 39])
@@ -85,6 +85,15 @@ def test_run_open_axis_repulsion(prec):
     """Harmonic repulsion with an open axis (the per-axis variant)."""
     sys_, xyz, types = plain(2000, per=(1, 1, 0))
     xc, xr, _ = both(prec, sys_, xyz, types, [130])
+    same(prec, xc, xr)
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+def test_run_small_batch(prec):
+    """Tiles that span systems, kept by their warps, across rebuilds."""
+    w = configs.config4(n_systems=12, nmin=200, nmax=3000)
+    xc, xr, nb = both(prec, w.system, w.xyz, w.types, [150, 1, 49], boxes=w.boxes, offsets=w.offsets)
+    assert nb > 3
     same(prec, xc, xr)
 
 
