@@ -135,9 +135,9 @@ typedef struct {
    graph_steps steps, times CELLS and LIST at skins of 0.1 .. 0.5 x rc_max on
    the handle's particles and keeps the fastest; the pair-list steps of an AUTO
    handle run many to a kernel launch, those of a LIST handle launch by launch
-   in captured graphs.  Every energy, force, digest
-   or RDF evaluation in LIST mode re-sorts and rebuilds the list (one build in
-   list_builds).                                                                */
+   in captured graphs.  Energies, forces and
+   digests in LIST mode are evaluated over the list, which holds every pair
+   within its cutoff between two calls.                                         */
 #define RDGPU_NB_AUTO  0
 #define RDGPU_NB_CELLS 1
 #define RDGPU_NB_LIST  2
@@ -158,8 +158,7 @@ typedef struct {
     int64_t  count[RDGPU_MAX_TYPES];    /* particles per type                        */
     int64_t  step;                      /* steps done since rdgpu_set_particles      */
     int32_t  neighbour_mode;            /* RDGPU_NB_CELLS or RDGPU_NB_LIST in effect */
-    int32_t  list_builds;               /* pair-list builds so far (before this call's
-                                           energy evaluation, which adds one)          */
+    int32_t  list_builds;               /* pair-list builds so far                  */
     double   skin;                      /* pair-list skin in effect [nm], 0: cells   */
     int32_t  list_capacity;             /* pair-list slots per particle              */
     int32_t  list_entry_bytes;          /* 2: partners as 16-bit offsets, 4: as 32-bit

@@ -157,6 +157,7 @@ struct rdgpu_engine {
     int nbuild_h = 0;
     int4* nbr = nullptr;                 // pair-list entry groups (narrow: 8 offsets, wide: 4 indices)
     uint2* head = nullptr;               // list heads: build position on a 16-bit lattice, list length
+    bool list_valid = false;             // the lists belong to the current state
     bool list_wide = false;              // 32-bit entries (a partner's offset did not fit 16 bits)
     int* hot = nullptr;                  // particles that moved more than about skin/2 since the build
     cudaStream_t stream2 = nullptr;      // captures the re-sort into conditional graph nodes
@@ -921,6 +922,7 @@ int read_back(Engine* E)
 template <class R> int resort(Engine* E, bool with_list)
 {
     if (E->npart_tot == 0) return RDGPU_OK;
+    E->list_valid = false;
     for (int attempt = 0; attempt < 16; ++attempt) {
         int rc = write_ctl(E, 1);
         if (rc) return rc;
@@ -934,7 +936,9 @@ template <class R> int resort(Engine* E, bool with_list)
         const int ef = *E->pinned_err;
         if (ef == 0) {
             set_cur(E, E->cur ^ 1);
-            return reset_counters(E, E->step_h);
+            rc = reset_counters(E, E->step_h);
+            E->list_valid = with_list && rc == RDGPU_OK;
+            return rc;
         }
         if (ef & ~(EF_LISTOVF | EF_LISTWIDE)) return fail(E, RDGPU_ERR_CUDA, "re-sort failed");
         // the scan cleared the counts; the current state is untouched
@@ -1193,8 +1197,19 @@ template <class R> int do_steps_list(Engine* E, long long nsteps, const double* 
     return RDGPU_OK;
 }
 
+// pair-list mode: lists of the current state (missing after a rejected edit
+// that had grown the buffers, or a failed re-sort)
+template <class R> int need_lists(Engine* E)
+{
+    if (E->nb_mode != RDGPU_NB_LIST || E->list_valid) return RDGPU_OK;
+    const int rc = ensure_list(E, list_cap_estimate(E), E->list_wide);
+    return rc ? rc : resort<R>(E, true);
+}
+
 template <class R> int do_steps_mode(Engine* E, long long nsteps, const double* noise_d)
 {
+    const int rc = need_lists<R>(E);
+    if (rc) return rc;
     return E->nb_mode == RDGPU_NB_LIST ? do_steps_list<R>(E, nsteps, noise_d) : do_steps_cells<R>(E, nsteps, noise_d);
 }
 
@@ -1471,7 +1486,10 @@ template <class R> int profile_list(Engine* E, long long nsteps, double* kms, do
 
 template <class R> int profile_impl(Engine* E, long long nsteps, double* kms, double* sms)
 {
-    if (E->nb_mode == RDGPU_NB_LIST) return profile_list<R>(E, nsteps, kms, sms);
+    if (E->nb_mode == RDGPU_NB_LIST) {
+        const int rc = need_lists<R>(E);
+        return rc ? rc : profile_list<R>(E, nsteps, kms, sms);
+    }
     ProfEvents pe;
     CK(pe.create());
     double tk = 0.0, ts = 0.0;
@@ -1639,6 +1657,7 @@ template <class R, class In> int set_particles_impl(Engine* E, const long long* 
     }
     if (ntot > 0x7fffffff) return fail(E, RDGPU_ERR_ARG, "at most 2^31-1 particles per handle");
     E->part_off.clear();   // no valid state until this call completes
+    E->list_valid = false;
     clear_bonds(E);        // bonds name particles of the previous upload
     if (ntot != E->npart_tot) drop_graphs(E);   // launch shapes depend on the particle count
     int rc = ensure_particle_buffers(E, ntot);
@@ -1765,6 +1784,7 @@ template <class R> int apply_edits_impl(Engine* E, const float* ed, long long co
     if (nd == 0 && na == 0) return RDGPU_OK;
     const long long nkeep = N - nd, N2 = nkeep + na;
     if (N2 > 0x7fffffff) return fail(E, RDGPU_ERR_ARG, "at most 2^31-1 particles per handle");
+    E->list_valid = false;
     int rc = grow_preserving<R>(E, N2);
     if (rc) { E->part_off.clear(); return rc; }
     drop_graphs(E);   // launch shapes depend on the particle count
@@ -1887,20 +1907,35 @@ template <class R> int sync_types(Engine* E)
     return RDGPU_OK;
 }
 
-template <class R, int MODE> void launch_diag(Engine* E, double* f, double* e, int* c, unsigned long long* h)
+// a walk over the cells in pair-list mode: re-sort first (the particles have
+// moved since the last build)
+template <class R> int fresh_cells(Engine* E)
 {
-    Args<R> a = make_args<R>(E);
+    return E->nb_mode == RDGPU_NB_LIST ? resort<R>(E, true) : RDGPU_OK;
+}
+
+// forces and energies (MODE 1) or neighbour digest (MODE 2) of the current
+// state: over the pair list where there is a valid one, else over the cells
+template <class R, int MODE> int launch_diag(Engine* E, double* f, double* e, int* c, unsigned long long* h)
+{
+    if (E->nb_mode == RDGPU_NB_LIST && E->list_valid) {
+        const Args<R> a = make_args<R>(E);
+        const ListArgs<R> v = make_list_args<R>(E, true);
+        const int grid = (int)((E->npart_tot + 127) / 128);
+        if (v.narrow)
+            diag_list_kernel<R, MODE, true><<<grid, 128, 0, E->stream>>>(a, v, f, e, c, h);
+        else
+            diag_list_kernel<R, MODE, false><<<grid, 128, 0, E->stream>>>(a, v, f, e, c, h);
+        return RDGPU_OK;
+    }
+    const int rc = fresh_cells<R>(E);
+    if (rc) return rc;
+    const Args<R> a = make_args<R>(E);
     if (E->value_image)
         diag_kernel<R, MODE, true><<<grid_for(E->npart_tot), 256, 0, E->stream>>>(a, f, e, c, h);
     else
         diag_kernel<R, MODE, false><<<grid_for(E->npart_tot), 256, 0, E->stream>>>(a, f, e, c, h);
-}
-
-// the diagnostics walk the cells: in pair-list mode re-sort first (the
-// particles have moved since the last build)
-template <class R> int fresh_cells(Engine* E)
-{
-    return E->nb_mode == RDGPU_NB_LIST ? resort<R>(E, true) : RDGPU_OK;
+    return RDGPU_OK;
 }
 
 // sums of v by type into red_d/redc_d: wants 0..nwant-1, type S meaning all
@@ -1916,9 +1951,8 @@ void launch_typed_sums(Engine* E, const double* v, const int* types, int S, int 
 
 template <class R> int forces_impl(Engine* E, double* forces, double* energy)
 {
-    int rc = fresh_cells<R>(E);
+    const int rc = launch_diag<R, 1>(E, E->vec_d, E->val_d, nullptr, nullptr);
     if (rc) return rc;
-    launch_diag<R, 1>(E, E->vec_d, E->val_d, nullptr, nullptr);
     CK(cudaGetLastError());
     if (forces) CK(cudaMemcpyAsync(forces, E->vec_d, E->npart_tot * 3 * sizeof(double), cudaMemcpyDeviceToHost, E->stream));
     if (energy) {
@@ -1932,9 +1966,8 @@ template <class R> int forces_impl(Engine* E, double* forces, double* energy)
 
 template <class R> int digest_impl(Engine* E, int* counts, unsigned long long* hashes)
 {
-    int rc = fresh_cells<R>(E);
+    const int rc = launch_diag<R, 2>(E, nullptr, nullptr, E->ityp_d, E->u64_d);
     if (rc) return rc;
-    launch_diag<R, 2>(E, nullptr, nullptr, E->ityp_d, E->u64_d);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(counts, E->ityp_d, E->npart_tot * sizeof(int), cudaMemcpyDeviceToHost, E->stream));
     CK(cudaMemcpyAsync(hashes, E->u64_d, E->npart_tot * sizeof(unsigned long long), cudaMemcpyDeviceToHost, E->stream));

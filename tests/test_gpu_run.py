@@ -140,3 +140,48 @@ def test_run_reports_a_failed_step(prec):
             x, _ = e.get_particles()
             assert np.isfinite(x).all()
     assert res[0] == res[1]
+
+
+def slab():
+    """200,000 particles whose neighbour cells lie more than 32,767 sorted places apart (32-bit list entries)."""
+    n = 200_000
+    sys_ = System([ParticleType("A", 1e6, 1.0)], pair=[PairPotential(A.P2_HARMONIC, [(0, 0)], 10.0, "repulsive")],
+                  kT=2.437, dt=1e-9, lo=(0, 0, 0), hi=(600, 600, 12), periodic=(1, 1, 1))
+    return sys_, np.random.default_rng(4).uniform((0, 0, 0), (600, 600, 12), (n, 3)), np.zeros(n, np.int32), 4
+
+
+@pytest.mark.parametrize("system", ["slab", "mixed", "lone"])
+def test_diagnostics_over_the_list(system):
+    """Forces, energy and neighbour sets evaluated over the list of a running
+    handle equal those of a cell walk of the same positions: 32- and 16-bit
+    entries, several terms per pair and an open axis, empty lists."""
+    if system == "slab":
+        sys_, xyz, types, width = slab()
+    elif system == "mixed":
+        sys_, xyz, types = small_config2(3000)
+        width = 2
+    else:
+        sys_, xyz, types = plain(40)
+        xyz, types, width = xyz[:1], types[:1], 2
+    with Engine(sys_, precision="f64", seed=3, neighbour_mode="list", skin=1.0) as e:
+        e.set_particles(xyz, types)
+        e.step(37)
+        x, t = e.get_particles()
+        F, en = e.forces()
+        cnt, h = e.neighbor_digest()
+        m = e.metrics()
+        assert m["list_entry_bytes"] == width and m["energy"] == en
+        with Engine(sys_, precision="f64", neighbour_mode="cells") as c:
+            c.set_particles(x, t)
+            Fc, enc = c.forces()
+            cntc, hc = c.neighbor_digest()
+        assert np.array_equal(cnt, cntc) and np.array_equal(h, hc)
+        assert np.linalg.norm(F - Fc) <= 1e-12 * np.linalg.norm(Fc)
+        assert abs(en - enc) <= 1e-10 * abs(enc)
+        # the evaluation leaves the run as it was
+        e.step(20)
+        y, _ = e.get_particles()
+    with Engine(sys_, precision="f64", seed=3, neighbour_mode="list", skin=1.0) as e:
+        e.set_particles(xyz, types)
+        e.step(57)
+        same("f64", e.get_particles()[0], y)
