@@ -131,8 +131,10 @@ typedef struct {
    more than about skin since the last build; after every step the particles
    that moved more than about skin/2 have their current neighbourhood
    checked against the list.  The pair set and the FP32 forces are identical
-   to CELLS.  AUTO starts with CELLS and, at the first rdgpu_step of >= 4 x
-   graph_steps steps, times CELLS and LIST at skins of 0.1 .. 0.5 x rc_max on
+   to CELLS.  AUTO starts with CELLS, times some 30 steps of it and 50 of LIST
+   (at a skin estimated from the diffusion constants) as it makes them and
+   keeps the faster; at the first rdgpu_step of >= 4 x graph_steps steps, or in
+   rdgpu_autotune, it times CELLS and LIST at skins of 0.1 .. 0.5 x rc_max on
    the handle's particles and keeps the fastest; the pair-list steps of an AUTO
    handle run many to a kernel launch, those of a LIST handle launch by launch
    in captured graphs.  Energies, forces and

@@ -185,3 +185,32 @@ def test_diagnostics_over_the_list(system):
         e.set_particles(xyz, types)
         e.step(57)
         same("f64", e.get_particles()[0], y)
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+@pytest.mark.parametrize("system,split", [("plain", [100, 40]), ("plain", [7] * 18), ("plain", [1] * 110),
+                                          ("mixed", [100]), ("small box", [100])])
+def test_untuned_handle_tries_the_list(prec, system, split):
+    """An AUTO handle that is never tuned and only gets short calls changes from
+    the cell walk to the pair list (and maybe back) within its first 100 steps;
+    the trajectory is the cell walk's.  A box too small for lists keeps the
+    cell walk."""
+    if system == "mixed":
+        sys_, xyz, types = small_config2(3000)
+    else:
+        sys_, xyz, types = plain(3000)
+        if system == "small box":
+            sys_.hi = (10.0, 10.0, 10.0)
+            xyz, types = xyz[:20] % 10.0, types[:20]
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision=prec, seed=4, neighbour_mode=mode) as e:
+            e.set_particles(xyz, types)
+            for n in split:
+                e.step(n)
+            m = e.metrics()
+            out.append(e.get_particles()[0])
+    assert m["step"] == sum(split)
+    if system == "small box":
+        assert m["neighbour_mode"] == "cells"
+    same(prec, out[0], out[1])
