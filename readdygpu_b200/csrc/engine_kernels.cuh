@@ -2319,54 +2319,54 @@ template <class R> struct ListCell {
     }
 };
 
-// The cells of row (dz, dy) around x that can hold a sorted particle closer
-// than sqrt(lim) to x: f(j0, j1, sx, sy, sz) for every range [j0, j1) of
-// sorted particles (two where the row wraps), with the periodic shift of its
-// cells.
-template <class R, class F>
-__device__ __forceinline__ void list_row_ranges(const Args<R>& a, const SysDev& s, const ListCell<R>& g, R lim,
-                                                int dz, int dy, F&& f)
+// Squared minimum-image distances of the list build: d = (xi - xj) - k L with
+// k = rint((xi - xj) / L), each operation rounded once.  Swapping i and j
+// negates every intermediate, so the test of a pair is the same from both
+// sides and j is in i's list exactly when i is in j's.
+template <class R> struct PairSym;
+template <> struct PairSym<float> {
+    f32x2 xy, il_xy, nl_xy;
+    float z, il_z, nl_z;
+    __device__ __forceinline__ void load(const SysDev& s, const float xi[3])
+    {
+        xy = f2_pack(xi[0], xi[1]);
+        il_xy = f2_pack(s.ilf[0], s.ilf[1]);
+        nl_xy = f2_pack(-s.Lf[0], -s.Lf[1]);
+        z = xi[2];
+        il_z = s.ilf[2];
+        nl_z = -s.Lf[2];
+    }
+};
+template <> struct PairSym<double> {
+    double x[3], il[3], nl[3];
+    __device__ __forceinline__ void load(const SysDev& s, const double xi[3])
+    {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) { x[a] = xi[a]; il[a] = s.il[a]; nl[a] = -s.L[a]; }
+    }
+};
+__device__ __forceinline__ float pair_dist2_sym(const PairSym<float>& f, const float xj[3])
 {
-    const R gz = gap2(dz, g.fr[2], g.cw[2]);
-    if (gz >= lim) return;
-    Box<R> bx;
-    bx.load(s);
-    const int n0 = s.n[0], n1 = s.n[1], n2 = s.n[2];
-    int z = g.c[2] + dz;
-    R sz = R(0);
-    if (z < 0 || z >= n2) {
-        if (!s.per[2]) return;
-        sz = z < 0 ? -bx.L[2] : bx.L[2];
-        z = z < 0 ? z + n2 : z - n2;
+    const float M = 12582912.0f;     // 1.5 2^23
+    const f32x2 t = f2_sub(f.xy, f2_pack(xj[0], xj[1]));
+    const f32x2 k = f2_add(f2_fma(t, f.il_xy, f2_pack(M, M)), f2_pack(-M, -M));
+    const f32x2 d = f2_fma(k, f.nl_xy, t);
+    float px, py;
+    f2_unpack(f2_mul(d, d), px, py);
+    const float tz = __fsub_rn(f.z, xj[2]);
+    const float dz = __fmaf_rn(__fadd_rn(__fmaf_rn(tz, f.il_z, M), -M), f.nl_z, tz);
+    return __fadd_rn(__fadd_rn(px, py), __fmul_rn(dz, dz));
+}
+__device__ __forceinline__ double pair_dist2_sym(const PairSym<double>& f, const double xj[3])
+{
+    const double M = 6755399441055744.0;   // 1.5 2^52
+    double d[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double t = __dsub_rn(f.x[a], xj[a]);
+        d[a] = __fma_rn(__dadd_rn(__fma_rn(t, f.il[a], M), -M), f.nl[a], t);
     }
-    const R gyz = gz + gap2(dy, g.fr[1], g.cw[1]);
-    if (gyz >= lim) return;
-    int y = g.c[1] + dy;
-    R sy = R(0);
-    if (y < 0 || y >= n1) {
-        if (!s.per[1]) return;
-        sy = y < 0 ? -bx.L[1] : bx.L[1];
-        y = y < 0 ? y + n1 : y - n1;
-    }
-    const int row = (int)s.cell_base + (z * n1 + y) * n0;
-    const R f0 = g.fr[0], w0 = g.cw[0];
-    int xa = (gyz + f0 * f0 < lim) ? g.c[0] - 1 : g.c[0];
-    int xb = (gyz + (w0 - f0) * (w0 - f0) < lim) ? g.c[0] + 1 : g.c[0];
-    const R L0 = bx.L[0];
-    if (!s.per[0]) {
-        xa = max(xa, 0);
-        xb = min(xb, n0 - 1);
-    } else {
-        if (xa < 0) {
-            f(a.start[row + n0 - 1], a.start[row + n0], -L0, sy, sz);
-            xa = 0;
-        }
-        if (xb >= n0) {
-            f(a.start[row], a.start[row + 1], L0, sy, sz);
-            xb = n0 - 1;
-        }
-    }
-    f(a.start[row + xa], a.start[row + xb + 1], R(0), sy, sz);
+    return dist2(d[0], d[1], d[2]);
 }
 
 // A thread's scratch for list_build_one, in shared memory (the words of one
@@ -2434,14 +2434,8 @@ __device__ __forceinline__ int list_build_one(const Args<R>& a, const ListArgs<R
     const R lim = v.rl2max * R(1.0001);
     const int n0 = s.n[0], n1 = s.n[1], n2 = s.n[2];
     const R fx2 = g.fr[0] * g.fr[0], gx2 = (g.cw[0] - g.fr[0]) * (g.cw[0] - g.fr[0]);
-    PairFrame pf;
-    R L[3] = {R(0), R(0), R(0)}, il[3] = {R(0), R(0), R(0)};
-    if constexpr (sizeof(R) == 4) {
-        pf.load(s, xi);
-    } else {
-#pragma unroll
-        for (int q = 0; q < 3; ++q) { L[q] = s.L[q]; il[q] = s.il[q]; }
-    }
+    PairSym<R> pf;
+    pf.load(s, xi);
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         int nr = 0, total = 0;
@@ -2489,14 +2483,7 @@ __device__ __forceinline__ int list_build_one(const Args<R>& a, const ListArgs<R
             for (int u = 0; u < CHUNK; ++u) load_pos<COH>(st, jj[u], xj[u], wj[u]);
 #pragma unroll
             for (int u = 0; u < CHUNK; ++u) {
-                R r2;
-                if constexpr (sizeof(R) == 4) {
-                    float dx, dy, dz;
-                    pair_disp_x2(pf, xj[u][0], xj[u][1], xj[u][2], dx, dy, dz, r2);
-                } else {
-                    r2 = dist2(mimg_round(xi[0], xj[u][0], L[0], il[0]), mimg_round(xi[1], xj[u][1], L[1], il[1]),
-                               mimg_round(xi[2], xj[u][2], L[2], il[2]));
-                }
+                const R r2 = pair_dist2_sym(pf, xj[u]);
                 if (r2 < rl2[wj[u] & 0xff] && jj[u] != i) {
                     ring[(cnt & (LB_RING - 1)) * B] = jj[u] - i;
                     ++cnt;
@@ -2541,24 +2528,14 @@ __global__ void __launch_bounds__(BLOCK) list_build_kernel(Args<R> a, ListArgs<R
     }
 }
 
-// j is in the pair list of i
-template <class R, bool COH>
-__device__ __forceinline__ bool listed(const ListArgs<R>& v, int i, int j)
-{
-    const int cnt = head_count(ld<COH>(v.head + i));
-    const int4* nb4 = v.nbr + i;
-    const int epg = v.narrow ? 8 : 4;
-    for (int k0 = 0; k0 < cnt; k0 += epg) {
-        const int4 q = ld<COH>(nb4 + (long long)(k0 / epg) * v.stride);
-        for (int u = 0; u < epg && k0 + u < cnt; ++u)
-            if (list_entry(q, u, v.narrow != 0, i) == j) return true;
-    }
-    return false;
-}
-
-// every particle now closer to hot particle h than their cutoff is in h's
-// list, and h in its; one warp per hot particle, lane r < 9 walks cell row r
-// of the 27-cell neighbourhood
+// Every particle now closer to hot particle h than their cutoff is in h's list
+// (and so h in its: the lists are symmetric, pair_dist2_sym).  One warp per
+// hot particle, a lane for each of the 27 cells around its current position.
+// Bound by latency, a chain of five loads: the hot list, h's state and first
+// list groups, its system, the cell's bounds, the candidates (4 at a time).
+// Against 9 lanes of a cell row each that looked pairs up in both lists, per
+// step in list_run_kernel (skin 1.4): 1,000 particles FP64 7.5 -> 6.4 us,
+// 20,000 FP64 8.7 -> 7.4, 1,000,000 FP32C 50.7 -> 48.2, 2.9 M 129 -> 125 us.
 template <class R, bool COH = false>
 __device__ __forceinline__ bool hot_pairs_listed(const Args<R>& a, const ListArgs<R>& v, const State<R>& st, int h,
                                                  int lane)
@@ -2567,33 +2544,51 @@ __device__ __forceinline__ bool hot_pairs_listed(const Args<R>& a, const ListArg
     R xh[3];
     int wh;
     load_pos<COH>(st, h, xh, wh);
+    const int cnt = head_count(ld<COH>(v.head + h));
+    const bool narrow = v.narrow != 0;
+    const int epg = narrow ? 8 : 4;
+    const int4 q0 = ld<COH>(v.nbr + h);
+    int c[3];
+    cell_coords(s, xh, c);
+    int q[3];
+    bool in = lane < 27;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        q[ax] = c[ax] + (ax == 0 ? lane % 3 : (ax == 1 ? (lane / 3) % 3 : lane / 9)) - 1;
+        if (q[ax] < 0 || q[ax] >= s.n[ax]) {
+            in = in && s.per[ax];
+            q[ax] += q[ax] < 0 ? s.n[ax] : -s.n[ax];
+        }
+    }
     bool ok = true;
-    if (lane < 9) {
+    if (in) {
         const R* rc2 = a.tab->rc2 + (wh & 0xff) * MAXT;
         Box<R> bx;
         bx.load(s);
-        ListCell<R> g;
-        g.locate(s, xh);
-        // candidates 4 at a time: their positions are requested together
-        // (past the range's end, its last candidate again, not tested)
-        list_row_ranges<R>(a, s, g, v.rl2max * R(1.0001), lane / 3 - 1, lane % 3 - 1, [&](int j0, int j1, R, R, R) {
-            for (int j = j0; j < j1 && ok; j += 4) {
-                R xj[4][3];
-                int wj[4];
+        const int cell = (int)s.cell_base + (q[2] * s.n[1] + q[1]) * s.n[0] + q[0];
+        const int j1 = a.start[cell + 1];
+        // (past the cell's end, its last candidate again, not tested)
+        for (int j = a.start[cell]; j < j1 && ok; j += 4) {
+            R xj[4][3];
+            int wj[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) load_pos<COH>(st, min(j + u, j1 - 1), xj[u], wj[u]);
+            for (int u = 0; u < 4; ++u) load_pos<COH>(st, min(j + u, j1 - 1), xj[u], wj[u]);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int jj = j + u;
-                    if (jj >= j1 || jj == h) continue;
-                    const R dx = mimg_sel(xh[0], xj[u][0], bx.L[0], bx.half[0], s.per[0]);
-                    const R dy = mimg_sel(xh[1], xj[u][1], bx.L[1], bx.half[1], s.per[1]);
-                    const R dz = mimg_sel(xh[2], xj[u][2], bx.L[2], bx.half[2], s.per[2]);
-                    if (dist2(dx, dy, dz) < rc2[wj[u] & 0xff] * R(1.0001) && !(listed<R, COH>(v, h, jj) && listed<R, COH>(v, jj, h)))
-                        ok = false;
+            for (int u = 0; u < 4; ++u) {
+                const int jj = j + u;
+                if (jj >= j1 || jj == h) continue;
+                const R dx = mimg_sel(xh[0], xj[u][0], bx.L[0], bx.half[0], s.per[0]);
+                const R dy = mimg_sel(xh[1], xj[u][1], bx.L[1], bx.half[1], s.per[1]);
+                const R dz = mimg_sel(xh[2], xj[u][2], bx.L[2], bx.half[2], s.per[2]);
+                if (!(dist2(dx, dy, dz) < rc2[wj[u] & 0xff] * R(1.0001))) continue;
+                bool found = false;
+                for (int k = 0; k < cnt && !found; k += epg) {
+                    const int4 g = k == 0 ? q0 : ld<COH>(v.nbr + (long long)(k / epg) * v.stride + h);
+                    for (int e = 0; e < epg && k + e < cnt; ++e) found |= list_entry(g, e, narrow, h) == jj;
                 }
+                ok = ok && found;
             }
-        });
+        }
     }
     return __all_sync(FULL, ok);
 }
@@ -2604,7 +2599,7 @@ __device__ __forceinline__ bool hot_pairs_listed(const Args<R>& a, const ListArg
 // particles moved by skin together since: one of them moved more than
 // sqrt(thr2) ~ skin/2 (a hot particle; the step kernel collects them).  For
 // every hot particle h, each particle now within its cutoff of h must be in
-// h's list and h in its.  The cell rows around h's current position reach
+// h's list (and so h in its).  The cells around h's current position reach
 // every such particle while no particle has moved more than sqrt(cap2) ~
 // skin since the build (the step kernel raises the rebuild flag itself
 // beyond that).  A missing pair, or more than hot_max hot particles, raise
