@@ -2115,12 +2115,11 @@ __device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>
     }, dd);
 }
 
-// collects the hot particles of a step (squared displacement dd above thr2)
-// and raises the rebuild flag beyond cap2
-__device__ __forceinline__ void list_collect_hot(float dd, float thr2, float cap2, int i, int* nhot, int* need,
-                                                 int* hot_list, int hot_max)
+// collects the hot particles of a step (squared displacement dd above thr2);
+// true in one lane of a warp that has any
+__device__ __forceinline__ bool list_collect_hot(float dd, float thr2, int i, int* nhot, int* hot_list, int hot_max)
 {
-    if (dd > cap2) *((volatile int*)need) = 1;
+    bool any = false;
     const bool hot = dd > thr2;
     const unsigned act = __activemask();
     const unsigned hm = __ballot_sync(act, hot);
@@ -2128,10 +2127,14 @@ __device__ __forceinline__ void list_collect_hot(float dd, float thr2, float cap
         const int lane = threadIdx.x & 31;
         const int lead = __ffs(hm) - 1;
         int base = 0;
-        if (lane == lead) base = atomicAdd(nhot, __popc(hm));
+        if (lane == lead) {
+            base = atomicAdd(nhot, __popc(hm));
+            any = true;
+        }
         base = __shfl_sync(act, base, lead) + __popc(hm & ((1u << lane) - 1u));
         if (hot && base < hot_max) hot_list[base] = i;
     }
+    return any;
 }
 
 // one BD step of every particle over its pair list; ALLPER: every axis of
@@ -2169,7 +2172,8 @@ __global__ void __launch_bounds__(BLOCK, (sizeof(R) == 4 ? (HREP && ALLPER ? 115
     if (!live) return;
     float dd;
     const int ef = list_step_one<R, HREP, ALLPER, NARROW, false>(a, v, cur, nxt, i, in, t, s_rc2, s_ft, s_one, dd);
-    list_collect_hot(dd, v.thr2, v.cap2, i, &v.ctl->nhot, &v.ctl->need, v.hot, v.hot_max);
+    if (dd > v.cap2) *((volatile int*)&v.ctl->need) = 1;
+    list_collect_hot(dd, v.thr2, i, &v.ctl->nhot, v.hot, v.hot_max);
     if (ef) {
         atomicOr(a.err, ef);
         atomicMin((unsigned long long*)a.err_step, (unsigned long long)t);
