@@ -1026,11 +1026,12 @@ template <class R> int capture_list_graph(Engine* E, int n, cudaGraphExec_t* out
     return RDGPU_OK;
 }
 
-template <class R> int launch_run_as(Engine* E, RunArgs<R>& p, const void* f, int block, int most, int grid)
+template <class R> int launch_run_as(Engine* E, RunArgs<R>& p, const void* f, int block, int grid, bool home)
 {
     void* args[] = {&p};
-    CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_dyn_bytes<R>(most)));
-    CK(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(block), args, run_dyn_bytes<R>(block), E->stream));
+    const size_t dyn = run_dyn_bytes<R>(block) + (home && !E->hrep ? run_term_bytes<R>(E->desc.n_types) : 0);
+    CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    CK(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(block), args, dyn, E->stream));
     ++E->launches;
     return RDGPU_OK;
 }
@@ -1041,6 +1042,7 @@ template <class R> int launch_run_as(Engine* E, RunArgs<R>& p, const void* f, in
 // up to the block's limit.
 template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E, RunArgs<R>& p)
 {
+    static_assert(MAX_EXT == RDGPU_MAX_EXT_POTS, "external potentials of a system in shared memory");
     const long long tiles = (E->npart_tot + 31) / 32;
     const int sms = E->sm_count;
     const int grid = (int)std::min<long long>(sms, tiles);
@@ -1048,14 +1050,15 @@ template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E
     if constexpr (NARROW) {
         if (per_sm <= RUN_HOME_FEW)
             return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_HOME_FEW>,
-                                 32 * ((int)per_sm + 4), run_home_block(RUN_HOME_FEW), grid);
+                                 32 * ((int)per_sm + 4), grid, true);
         if (per_sm <= RUN_HOME_MANY)
             return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_HOME_MANY>,
-                                 32 * ((int)per_sm + 3), run_home_block(RUN_HOME_MANY), grid);
+                                 32 * ((int)per_sm + 3), grid, true);
     }
     constexpr int most = RunShape<R, HREP, ALLPER>::BLOCK;
     const int block = 32 * (int)std::max<long long>(4, std::min<long long>(most / 32, per_sm));
-    return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, NARROW, 0>, block, most, grid);
+    return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, NARROW, 0>, block, grid,
+                         false);
 }
 
 template <class R, bool NARROW> int launch_run_w(Engine* E, RunArgs<R>& p, bool allper)

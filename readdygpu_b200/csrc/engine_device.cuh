@@ -21,6 +21,7 @@ namespace rdgpu {
 
 constexpr int MAXT = 16;
 constexpr int MAX_TERMS = 4;
+constexpr int MAX_EXT = 16;
 constexpr unsigned FULL = 0xffffffffu;
 
 // error flags

@@ -1955,28 +1955,34 @@ template <class R, bool NARROW, bool COH> struct ListIn {
     }
 };
 
-// The pair tables of a block: rows of the S types in use (entries (ti, tj)
-// with ti >= S are never read).  one[]: the pair has at most one term, a
-// harmonic repulsion (k, r0 in the FastTab; with HREP every pair has).
-template <class R, bool HREP>
-__device__ __forceinline__ void load_pair_tables(const TypeTab<R>* tab, R* s_rc2, FastTab<R>& s_ft, bool* s_one)
-{
-    for (int k = threadIdx.x; k < MAXT * tab->S; k += blockDim.x) {
-        s_rc2[k] = tab->rc2[k];
-        const PairTerm<R>& t = tab->term[k * MAX_TERMS];
-        s_ft.k[k] = tab->nterm[k] ? t.k : R(0);
-        s_ft.r0[k] = tab->nterm[k] ? t.r0 : R(0);
-        if (!HREP) s_one[k] = tab->nterm[k] <= 1 && t.kind == 1 && t.sub == 2;
+// The pair tables of a block in shared memory: rows of the S types in use
+// (entries (ti, tj) with ti >= S are never read).  Without HREP, one[] says
+// that the pair has at most one term, a harmonic repulsion (its k and r0 are
+// in ft; with HREP every pair has).
+template <class R, bool HREP> struct PairTables {
+    R rc2[MAXT * MAXT];
+    FastTab<R> ft;
+    bool one[HREP ? 1 : MAXT * MAXT];
+    __device__ __forceinline__ void load(const TypeTab<R>* tab)
+    {
+        for (int k = threadIdx.x; k < MAXT * tab->S; k += blockDim.x) {
+            rc2[k] = tab->rc2[k];
+            const PairTerm<R>& t = tab->term[k * MAX_TERMS];
+            ft.k[k] = tab->nterm[k] ? t.k : R(0);
+            ft.r0[k] = tab->nterm[k] ? t.r0 : R(0);
+            if (!HREP) one[k] = tab->nterm[k] <= 1 && t.kind == 1 && t.sub == 2;
+        }
     }
-}
+};
 
 // The pair forces on particle i over its list.  LCHUNK: entries whose positions
-// are requested together; SECOND: the second narrow group is in in.q1.
+// are requested together; SECOND: the second narrow group is in in.q1.  Pairs
+// of several terms take entry ti tstride + tj of nterm and terms.
 template <class R, bool HREP, bool NARROW, bool COH, int LCHUNK, bool SECOND>
 __device__ __forceinline__ void list_pairs(const Args<R>& a, const ListArgs<R>& v, const State<R>& cur, int i,
                                            const ListIn<R, NARROW, COH>& in, const SysDev& s,
-                                           const R* __restrict__ s_rc2, const FastTab<R>& s_ft,
-                                           const bool* __restrict__ s_one, Acc<R>& acc)
+                                           const PairTables<R, HREP>& pt, const int* nterm,
+                                           const PairTerm<R>* terms, int tstride, Acc<R>& acc)
 {
     const R* xi = in.xi;
     const int ti = in.wi & 0xff;
@@ -2035,27 +2041,28 @@ __device__ __forceinline__ void list_pairs(const Args<R>& a, const ListArgs<R>& 
                 r2 = dist2(dx, dy, dz);
             }
             const int pidx = ti * MAXT + (wj[u] & 0xff);
-            if (r2 < s_rc2[pidx]) {
+            if (r2 < pt.rc2[pidx]) {
                 if (HREP) {
                     // pre = k (r - r0) / r; r == 0 has no direction
                     if (r2 > R(0)) {
                         R pre;
-                        if constexpr (sizeof(R) == 4) pre = s_ft.k[pidx] * (1.0f - s_ft.r0[pidx] * rsqrtf(r2));
-                        else { const R r = sqrt(r2); pre = s_ft.k[pidx] * (r - s_ft.r0[pidx]) / r; }
+                        if constexpr (sizeof(R) == 4) pre = pt.ft.k[pidx] * (1.0f - pt.ft.r0[pidx] * rsqrtf(r2));
+                        else { const R r = sqrt(r2); pre = pt.ft.k[pidx] * (r - pt.ft.r0[pidx]) / r; }
                         acc.add(pre, dx, dy, dz);
                     }
                 } else if (r2 > R(0)) {
                     // (a coincident pair has no direction: every term times
                     // a zero displacement)
                     const R r = sqrt(r2);
-                    if (s_one[pidx]) {
-                        const R r0 = s_ft.r0[pidx];
-                        if (r < r0) acc.add(s_ft.k[pidx] * (r - r0) / r, dx, dy, dz);
+                    if (pt.one[pidx]) {
+                        const R r0 = pt.ft.r0[pidx];
+                        if (r < r0) acc.add(pt.ft.k[pidx] * (r - r0) / r, dx, dy, dz);
                     } else {
-                        const int nt = a.tab->nterm[pidx];
+                        const int q = ti * tstride + (wj[u] & 0xff);
+                        const int nt = nterm[q];
                         for (int m = 0; m < nt; ++m) {
                             R pre, e;
-                            pair_term(a.tab->term[pidx * MAX_TERMS + m], r, pre, e);
+                            pair_term(terms[q * MAX_TERMS + m], r, pre, e);
                             acc.add(pre, dx, dy, dz);
                         }
                     }
@@ -2069,10 +2076,11 @@ __device__ __forceinline__ void list_pairs(const Args<R>& a, const ListArgs<R>& 
 // by noise() last, when the fewest registers are held): the new state to in
 // and to nxt; returns the error flags and, in dd, the squared displacement
 // since the build (lattice estimate; the thresholds allow for its error).
+// ext: the external potentials of i's system.
 template <class R, bool ALLPER, bool NARROW, bool COH, class N>
 __device__ __forceinline__ int list_move(const Args<R>& a, const State<R>& cur, const State<R>& nxt, int i,
-                                         ListIn<R, NARROW, COH>& in, const SysDev& s, Acc<R>& acc, N&& noise,
-                                         float& dd)
+                                         ListIn<R, NARROW, COH>& in, const SysDev& s, Acc<R>& acc,
+                                         const ExtTerm<R>* ext, N&& noise, float& dd)
 {
     R* xi = in.xi;
     const int ti = in.wi & 0xff;
@@ -2080,10 +2088,9 @@ __device__ __forceinline__ int list_move(const Args<R>& a, const State<R>& cur, 
     R F[3];
     acc.force(F);
     if (a.n_ext > 0) {
-        const ExtTerm<R>* ep = a.ext + (long long)in.si * a.n_ext;
         R ee = R(0);
         for (int e = 0; e < a.n_ext; ++e)
-            if ((ep[e].tmask >> ti) & 1u) ext_force(ep[e], a.tab->prad[ti], xi, F, ee);
+            if ((ext[e].tmask >> ti) & 1u) ext_force(ext[e], a.tab->prad[ti], xi, F, ee);
     }
     R xn[3];
     noise(xn);
@@ -2097,15 +2104,15 @@ __device__ __forceinline__ int list_move(const Args<R>& a, const State<R>& cur, 
 template <class R, bool HREP, bool ALLPER, bool NARROW, bool COH>
 __device__ __forceinline__ int list_step_one(const Args<R>& a, const ListArgs<R>& v, const State<R>& cur,
                                              const State<R>& nxt, int i, ListIn<R, NARROW, COH>& in, long long t,
-                                             const R* __restrict__ s_rc2, const FastTab<R>& s_ft,
-                                             const bool* __restrict__ s_one, float& dd)
+                                             const PairTables<R, HREP>& pt, const int* nterm,
+                                             const PairTerm<R>* terms, int tstride, const ExtTerm<R>* ext, float& dd)
 {
     const SysDev& s = a.sys[in.si];
     Acc<R> acc;
     acc.zero();
-    list_pairs<R, HREP, NARROW, COH, sizeof(R) == 4 ? LIST_CHUNK : LIST_CHUNK_F64, false>(a, v, cur, i, in, s, s_rc2,
-                                                                                          s_ft, s_one, acc);
-    return list_move<R, ALLPER>(a, cur, nxt, i, in, s, acc, [&](R* xn) {
+    list_pairs<R, HREP, NARROW, COH, sizeof(R) == 4 ? LIST_CHUNK : LIST_CHUNK_F64, false>(a, v, cur, i, in, s, pt,
+                                                                                          nterm, terms, tstride, acc);
+    return list_move<R, ALLPER>(a, cur, nxt, i, in, s, acc, ext, [&](R* xn) {
         if (a.noise) {
             const double* nz = a.noise + 3 * (s.part_base + in.id);
             xn[0] = (R)nz[0]; xn[1] = (R)nz[1]; xn[2] = (R)nz[2];
@@ -2149,9 +2156,7 @@ __global__ void __launch_bounds__(BLOCK, (sizeof(R) == 4 ? (HREP && ALLPER ? 115
                                              BLOCK)
     list_step_kernel(Args<R> a, ListArgs<R> v)
 {
-    __shared__ R s_rc2[MAXT * MAXT];
-    __shared__ FastTab<R> s_ft;
-    __shared__ bool s_one[HREP ? 1 : MAXT * MAXT];
+    __shared__ PairTables<R, HREP> s_pt;
     // the error flag, the step counter and the buffer parity, then the
     // particle's inputs, all requested before the pair tables: the block
     // waits on one round of loads, not three
@@ -2167,11 +2172,12 @@ __global__ void __launch_bounds__(BLOCK, (sizeof(R) == 4 ? (HREP && ALLPER ? 115
     ListIn<R, NARROW, false> in;
     in.clear();
     if (live) in.load(a, v, cur, i);
-    load_pair_tables<R, HREP>(a.tab, s_rc2, s_ft, s_one);
+    s_pt.load(a.tab);
     __syncthreads();
     if (!live) return;
     float dd;
-    const int ef = list_step_one<R, HREP, ALLPER, NARROW, false>(a, v, cur, nxt, i, in, t, s_rc2, s_ft, s_one, dd);
+    const int ef = list_step_one<R, HREP, ALLPER, NARROW, false>(
+        a, v, cur, nxt, i, in, t, s_pt, a.tab->nterm, a.tab->term, MAXT, a.ext + (long long)in.si * a.n_ext, dd);
     if (dd > v.cap2) *((volatile int*)&v.ctl->need) = 1;
     list_collect_hot(dd, v.thr2, i, &v.ctl->nhot, v.hot, v.hot_max);
     if (ef) {

@@ -77,9 +77,17 @@ constexpr unsigned RUN_POLLS = 1u << 23;
 
 constexpr int RUN_SCAN_PER = 8;       // cells per thread and scan tile
 
-// dynamic shared memory: the squared list radii, then list_build_one's scratch
+// dynamic shared memory: the squared list radii, list_build_one's scratch, then
+// (HOME without HREP) the terms of the type pairs in use
 extern __shared__ __align__(16) char run_dyn[];
-template <class R> constexpr size_t run_dyn_bytes(int block) { return MAXT * MAXT * sizeof(R) + (size_t)block * LB_BYTES; }
+template <class R> __host__ __device__ constexpr size_t run_dyn_bytes(int block)
+{
+    return MAXT * MAXT * sizeof(R) + (size_t)block * LB_BYTES;
+}
+template <class R> constexpr size_t run_term_bytes(int S)
+{
+    return (size_t)((S * S + 3) & ~3) * sizeof(int) + (size_t)S * S * MAX_TERMS * sizeof(PairTerm<R>);
+}
 
 __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p)
 {
@@ -355,9 +363,8 @@ template <class R, bool HREP, bool ALLPER, bool NARROW, int HOME>
 __global__ void __launch_bounds__(HOME ? run_home_block(HOME) : RunShape<R, HREP, ALLPER>::BLOCK, 1)
     list_run_kernel(const __grid_constant__ RunArgs<R> p)
 {
-    __shared__ R s_rc2[MAXT * MAXT];
-    __shared__ FastTab<R> s_ft;
-    __shared__ bool s_one[HREP ? 1 : MAXT * MAXT];
+    __shared__ PairTables<R, HREP> s_pt;
+    __shared__ __align__(16) char s_ext[HOME > 0 ? MAX_EXT * sizeof(ExtTerm<R>) : 16];
     __shared__ RunShared sh;
     const Args<R>& a = p.a;
     const ListArgs<R>& v = p.v;
@@ -370,7 +377,26 @@ __global__ void __launch_bounds__(HOME ? run_home_block(HOME) : RunShape<R, HREP
         sh.mine = 0;
         sh.next = blockDim.x >> 5;
     }
-    load_pair_tables<R, HREP>(a.tab, s_rc2, s_ft, s_one);
+    s_pt.load(a.tab);
+    // HOME: the terms of the type pairs in use and a single system's external
+    // potentials too, since a barrier drops L1 and each step would wait for
+    // them anew (60,000 particles FP64, vesicle: 18.1 -> 16.7 us a step; with
+    // many tiles per warp the plain loads measured 2 to 6 % faster)
+    const int S = a.tab->S;
+    int* s_nterm = reinterpret_cast<int*>(run_dyn + run_dyn_bytes<R>(blockDim.x));
+    PairTerm<R>* s_term = reinterpret_cast<PairTerm<R>*>(s_nterm + ((S * S + 3) & ~3));
+    const ExtTerm<R>* ext1 = reinterpret_cast<const ExtTerm<R>*>(s_ext);
+    if constexpr (HOME > 0) {
+        if (!HREP)
+            for (int q = threadIdx.x; q < S * S; q += blockDim.x) {
+                const int k = (q / S) * MAXT + q % S;
+                s_nterm[q] = a.tab->nterm[k];
+                for (int m = 0; m < MAX_TERMS; ++m) s_term[q * MAX_TERMS + m] = a.tab->term[k * MAX_TERMS + m];
+            }
+        if (a.nsys == 1)
+            for (int q = threadIdx.x; q < a.n_ext * (int)(sizeof(ExtTerm<R>) / 4); q += blockDim.x)
+                reinterpret_cast<int*>(s_ext)[q] = reinterpret_cast<const int*>(a.ext)[q];
+    }
     __syncthreads();
     long long t = p.t0;
     int sel = p.sel0, n = 0, slot = 0, builds = 0, nhot = 0, err = 0;
@@ -408,10 +434,11 @@ __global__ void __launch_bounds__(HOME ? run_home_block(HOME) : RunShape<R, HREP
                 }
                 Acc<R> acc;
                 acc.zero();
-                list_pairs<R, HREP, NARROW, true, RUN_HOME_CHUNK<R>, true>(a, v, cur, hi, hin, hs, s_rc2, s_ft,
-                                                                                          s_one, acc);
+                list_pairs<R, HREP, NARROW, true, RUN_HOME_CHUNK<R>, true>(a, v, cur, hi, hin, hs, s_pt, s_nterm,
+                                                                           s_term, S, acc);
                 float dd;
-                const int ef = list_move<R, ALLPER>(a, cur, nxt, hi, hin, hs, acc, [&](R* xn) {
+                const int ef = list_move<R, ALLPER>(a, cur, nxt, hi, hin, hs, acc,
+                                                    a.nsys == 1 ? ext1 : a.ext + (long long)hin.si * a.n_ext, [&](R* xn) {
                     xn[0] = hn[0]; xn[1] = hn[1]; xn[2] = hn[2];
                 }, dd);
                 const bool any = list_collect_hot(dd, v.thr2, hi, &p.ctl->nhot[slot], hot_out, v.hot_max);
@@ -436,8 +463,9 @@ __global__ void __launch_bounds__(HOME ? run_home_block(HOME) : RunShape<R, HREP
                     ListIn<R, NARROW, true> in;
                     in.load(a, v, cur, i);
                     float dd;
-                    const int ef = list_step_one<R, HREP, ALLPER, NARROW, true>(a, v, cur, nxt, i, in, t, s_rc2, s_ft,
-                                                                                   s_one, dd);
+                    const int ef = list_step_one<R, HREP, ALLPER, NARROW, true>(
+                        a, v, cur, nxt, i, in, t, s_pt, a.tab->nterm, a.tab->term, MAXT,
+                        a.ext + (long long)in.si * a.n_ext, dd);
                     const bool any = list_collect_hot(dd, v.thr2, i, &p.ctl->nhot[slot], hot_out, v.hot_max);
                     if (ef) atomicOr(&p.ctl->err[slot], ef);
                     if (any || ef || dd > v.cap2)
