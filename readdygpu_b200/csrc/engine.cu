@@ -1039,7 +1039,8 @@ template <class R> int launch_run_as(Engine* E, RunArgs<R>& p, const void* f, in
 // list_run_kernel with one block per SM: up to RUN_HOME_MANY tiles of 32
 // particles per SM, a warp per tile that keeps it and the rest of the block for
 // the hot particles (narrow lists); beyond that a warp per tile that an SM gets,
-// up to the block's limit.
+// up to the block's limit, and with more tiles than that in the order of their
+// cost where it differs (RUN_RANK).
 template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E, RunArgs<R>& p)
 {
     static_assert(MAX_EXT == RDGPU_MAX_EXT_POTS, "external potentials of a system in shared memory");
@@ -1057,6 +1058,10 @@ template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E
     }
     constexpr int most = RunShape<R, HREP, ALLPER>::BLOCK;
     const int block = 32 * (int)std::max<long long>(4, std::min<long long>(most / 32, per_sm));
+    if constexpr (NARROW && !HREP) {
+        if (per_sm > most / 32)
+            return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_RANK>, block, grid, false);
+    }
     return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, NARROW, 0>, block, grid,
                          false);
 }

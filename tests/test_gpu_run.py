@@ -214,3 +214,13 @@ def test_untuned_handle_tries_the_list(prec, system, split):
     if system == "small box":
         assert m["neighbour_mode"] == "cells"
     same(prec, out[0], out[1])
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+def test_run_tiles_in_the_order_of_their_cost(prec):
+    """Several tiles per warp and several potentials (the ordered variant),
+    across rebuilds and calls: the vesicle."""
+    w = configs.config5(n=160_000)
+    xc, xr, nb = both(prec, w.system, w.xyz, w.types, [40, 1, 19])
+    assert nb > 1
+    same(prec, xc, xr)
