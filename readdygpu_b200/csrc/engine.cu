@@ -14,6 +14,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <unordered_set>
 #include <vector>
 
 #include "../../include/readdy_b200.h"
@@ -41,6 +42,8 @@ constexpr int kCheckBlock = 256;
 constexpr int kCheckBlocks = 512;
 // steps of one list_run_kernel launch, at most
 constexpr long long kRunSteps = 1024;
+constexpr const char* kBadInput = "particle type out of range, non-finite coordinate, or a coordinate more than 64 box "
+                                  "lengths outside the box";
 }  // namespace
 
 std::string& rdgpu_global_error() { return g_create_error; }
@@ -920,13 +923,115 @@ int read_back(Engine* E)
     return RDGPU_OK;
 }
 
+template <class R> int launch_run_as(Engine* E, RunArgs<R>& p, const void* f, int block, int grid, bool home)
+{
+    void* args[] = {&p};
+    const size_t dyn = run_dyn_bytes<R>(block) + (home && !E->hrep ? run_term_bytes<R>(E->desc.n_types) : 0);
+    CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    CK(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(block), args, dyn, E->stream));
+    ++E->launches;
+    return RDGPU_OK;
+}
+
+// list_run_kernel with one block per SM: up to RUN_HOME_MANY tiles of 32
+// particles per SM, a warp per tile that keeps it and the rest of the block for
+// the hot particles (narrow lists); beyond that a warp per tile that an SM gets,
+// up to the block's limit, and with more tiles than that in the order of their
+// cost where it differs (RUN_RANK).
+template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E, RunArgs<R>& p)
+{
+    static_assert(MAX_EXT == RDGPU_MAX_EXT_POTS, "external potentials of a system in shared memory");
+    const long long tiles = (E->npart_tot + 31) / 32;
+    const int sms = E->sm_count;
+    const int grid = (int)std::min<long long>(sms, tiles);
+    const long long per_sm = (tiles + grid - 1) / grid;
+    if constexpr (NARROW) {
+        if (per_sm <= RUN_HOME_FEW)
+            return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_HOME_FEW>,
+                                 32 * ((int)per_sm + 4), grid, true);
+        if (per_sm <= RUN_HOME_MANY)
+            return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_HOME_MANY>,
+                                 32 * ((int)per_sm + 3), grid, true);
+    }
+    constexpr int most = RunShape<R, HREP, ALLPER>::BLOCK;
+    const int block = 32 * (int)std::max<long long>(4, std::min<long long>(most / 32, per_sm));
+    if constexpr (NARROW && !HREP) {
+        if (per_sm > most / 32)
+            return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_RANK>, block, grid, false);
+    }
+    return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, NARROW, 0>, block, grid,
+                         false);
+}
+
+template <class R, bool NARROW> int launch_run_w(Engine* E, RunArgs<R>& p, bool allper)
+{
+    if (E->hrep) return allper ? launch_run<R, true, true, NARROW>(E, p) : launch_run<R, true, false, NARROW>(E, p);
+    return allper ? launch_run<R, false, true, NARROW>(E, p) : launch_run<R, false, false, NARROW>(E, p);
+}
+
+// one launch of up to n pair-list steps from step step_h (rebuild: RUN_REBUILD*,
+// after a re-sort and list build); waits for it
+template <class R> int run_steps(Engine* E, int n, int rebuild = 0)
+{
+    // scan tiles of the smallest block
+    const long long nt = E->ncells_tot / (128 * RUN_SCAN_PER) + 2;
+    if (nt > E->run_tsum_n) {
+        dfree(E->run_tsum);
+        E->run_tsum_n = 0;
+        CK(cudaMalloc(&E->run_tsum, nt * sizeof(int)));
+        E->run_tsum_n = nt;
+    }
+    RunArgs<R> p;
+    memset(&p, 0, sizeof(p));
+    p.a = make_args<R>(E);
+    p.v = make_list_args<R>(E, true);
+    p.ctl = E->run_ctl + E->run_k;
+    p.next = E->run_ctl + (E->run_k ^ 1);
+    p.out = E->run_out;
+    p.tile_sum = E->run_tsum;
+    p.ncells = E->ncells_tot;
+    p.t0 = E->step_h;
+    p.nsteps = n;
+    p.sel0 = E->cur;
+    p.rebuild = rebuild;
+    const int rc = p.v.narrow ? launch_run_w<R, true>(E, p, all_periodic(E)) : launch_run_w<R, false>(E, p, all_periodic(E));
+    if (rc) return rc;
+    E->run_k ^= 1;
+    CK(cudaStreamSynchronize(E->stream));
+    return RDGPU_OK;
+}
+
 // Re-sorts the current state (the input of step step_h) by cell into the
 // other buffer and, with_list, builds the pair lists; an overflowing build
 // grows the lists and is redone.
-template <class R> int resort(Engine* E, bool with_list)
+// check_input: the state comes from an upload that the kernels may have
+// rejected (RDGPU_ERR_ARG then).
+template <class R> int resort(Engine* E, bool with_list, bool check_input = false)
 {
     if (E->npart_tot == 0) return RDGPU_OK;
     E->list_valid = false;
+    if (with_list && run_in_one(E)) {
+        // all of it in one launch and one wait (chain of launches: six, and
+        // three waits; 20,000 particles FP64 171 -> 99 us per upload)
+        for (int attempt = 0; attempt < 16; ++attempt) {
+            int rc = run_steps<R>(E, 0, check_input ? RUN_REBUILD_INPUT : RUN_REBUILD);
+            if (rc) return rc;
+            const RunOut o = *E->run_out;
+            if (o.dead) return fail(E, RDGPU_ERR_CUDA, "a grid barrier of the list build timed out");
+            if (o.err & EF_BADINPUT) return fail(E, RDGPU_ERR_ARG, kBadInput);
+            if (o.err == 0) {
+                set_cur(E, o.sel);
+                E->nbuild_h += o.builds;
+                E->list_valid = true;
+                return RDGPU_OK;
+            }
+            if (o.err & ~(EF_LISTOVF | EF_LISTWIDE)) return fail(E, RDGPU_ERR_CUDA, "re-sort failed");
+            E->pinned_ctl->maxcnt = o.maxcnt;
+            rc = ensure_list_after(E, o.err);
+            if (rc) return rc;
+        }
+        return fail(E, RDGPU_ERR_CUDA, "pair-list build did not converge");
+    }
     for (int attempt = 0; attempt < 16; ++attempt) {
         int rc = write_ctl(E, 1);
         if (rc) return rc;
@@ -1023,82 +1128,6 @@ template <class R> int capture_list_graph(Engine* E, int n, cudaGraphExec_t* out
     CK(ie);
     E->lgraphs[n] = x;
     *out = x;
-    return RDGPU_OK;
-}
-
-template <class R> int launch_run_as(Engine* E, RunArgs<R>& p, const void* f, int block, int grid, bool home)
-{
-    void* args[] = {&p};
-    const size_t dyn = run_dyn_bytes<R>(block) + (home && !E->hrep ? run_term_bytes<R>(E->desc.n_types) : 0);
-    CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    CK(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(block), args, dyn, E->stream));
-    ++E->launches;
-    return RDGPU_OK;
-}
-
-// list_run_kernel with one block per SM: up to RUN_HOME_MANY tiles of 32
-// particles per SM, a warp per tile that keeps it and the rest of the block for
-// the hot particles (narrow lists); beyond that a warp per tile that an SM gets,
-// up to the block's limit, and with more tiles than that in the order of their
-// cost where it differs (RUN_RANK).
-template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E, RunArgs<R>& p)
-{
-    static_assert(MAX_EXT == RDGPU_MAX_EXT_POTS, "external potentials of a system in shared memory");
-    const long long tiles = (E->npart_tot + 31) / 32;
-    const int sms = E->sm_count;
-    const int grid = (int)std::min<long long>(sms, tiles);
-    const long long per_sm = (tiles + grid - 1) / grid;
-    if constexpr (NARROW) {
-        if (per_sm <= RUN_HOME_FEW)
-            return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_HOME_FEW>,
-                                 32 * ((int)per_sm + 4), grid, true);
-        if (per_sm <= RUN_HOME_MANY)
-            return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_HOME_MANY>,
-                                 32 * ((int)per_sm + 3), grid, true);
-    }
-    constexpr int most = RunShape<R, HREP, ALLPER>::BLOCK;
-    const int block = 32 * (int)std::max<long long>(4, std::min<long long>(most / 32, per_sm));
-    if constexpr (NARROW && !HREP) {
-        if (per_sm > most / 32)
-            return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_RANK>, block, grid, false);
-    }
-    return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, NARROW, 0>, block, grid,
-                         false);
-}
-
-template <class R, bool NARROW> int launch_run_w(Engine* E, RunArgs<R>& p, bool allper)
-{
-    if (E->hrep) return allper ? launch_run<R, true, true, NARROW>(E, p) : launch_run<R, true, false, NARROW>(E, p);
-    return allper ? launch_run<R, false, true, NARROW>(E, p) : launch_run<R, false, false, NARROW>(E, p);
-}
-
-// one launch of up to n pair-list steps from step step_h; waits for it
-template <class R> int run_steps(Engine* E, int n)
-{
-    // scan tiles of the smallest block
-    const long long nt = E->ncells_tot / (128 * RUN_SCAN_PER) + 2;
-    if (nt > E->run_tsum_n) {
-        dfree(E->run_tsum);
-        E->run_tsum_n = 0;
-        CK(cudaMalloc(&E->run_tsum, nt * sizeof(int)));
-        E->run_tsum_n = nt;
-    }
-    RunArgs<R> p;
-    memset(&p, 0, sizeof(p));
-    p.a = make_args<R>(E);
-    p.v = make_list_args<R>(E, true);
-    p.ctl = E->run_ctl + E->run_k;
-    p.next = E->run_ctl + (E->run_k ^ 1);
-    p.out = E->run_out;
-    p.tile_sum = E->run_tsum;
-    p.ncells = E->ncells_tot;
-    p.t0 = E->step_h;
-    p.nsteps = n;
-    p.sel0 = E->cur;
-    const int rc = p.v.narrow ? launch_run_w<R, true>(E, p, all_periodic(E)) : launch_run_w<R, false>(E, p, all_periodic(E));
-    if (rc) return rc;
-    E->run_k ^= 1;
-    CK(cudaStreamSynchronize(E->stream));
     return RDGPU_OK;
 }
 
@@ -1737,6 +1766,8 @@ template <class R, class In> int set_particles_impl(Engine* E, const long long* 
         E->sys_h[s].npart = (int)(off[s + 1] - off[s]);
     }
     E->npart_tot = ntot;
+    const bool list_mode = E->nb_mode == RDGPU_NB_LIST && ntot > 0;
+    const bool one = list_mode && run_in_one(E);   // the list build checks the input itself: one wait
     CK(cudaMemcpyAsync(E->sys_d, E->sys_h.data(), E->nsys * sizeof(SysDev), cudaMemcpyHostToDevice, E->stream));
     CK(cudaMemsetAsync(E->err, 0, sizeof(int), E->stream));
     CK(cudaMemsetAsync(E->counts, 0, std::max<long long>(E->ncells_tot, 1) * sizeof(int), E->stream));
@@ -1750,19 +1781,18 @@ template <class R, class In> int set_particles_impl(Engine* E, const long long* 
                                                                 E->desc.n_types, stg_state<R>(E),
                                                                 E->tcell, E->tslot, E->counts, E->x0_d, E->err);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(E->pinned_err, E->err, sizeof(int), cudaMemcpyDeviceToHost, E->stream));
-        CK(cudaStreamSynchronize(E->stream));
-        if (*E->pinned_err & EF_BADINPUT)
-            return fail(E, RDGPU_ERR_ARG, "particle type out of range, non-finite coordinate, or a coordinate "
-                                          "more than 64 box lengths outside the box");
+        if (!one) {
+            CK(cudaMemcpyAsync(E->pinned_err, E->err, sizeof(int), cudaMemcpyDeviceToHost, E->stream));
+            CK(cudaStreamSynchronize(E->stream));
+            if (*E->pinned_err & EF_BADINPUT) return fail(E, RDGPU_ERR_ARG, kBadInput);
+        }
     }
     // the host copy of the types is downloaded when needed (sync_types)
     E->types_h_valid = false;
-    const bool list_mode = E->nb_mode == RDGPU_NB_LIST && ntot > 0;
     if (list_mode) {
         // the list re-sort below sorts the ingested particles itself: the
         // staging buffer becomes the current state (its counts are cleared
-        // by prepare_step_state)
+        // below)
         set_cur(E, E->cur ^ 1);
     } else {
         launch_sort<R>(E);
@@ -1773,12 +1803,17 @@ template <class R, class In> int set_particles_impl(Engine* E, const long long* 
         const int S = E->desc.n_types;
         CK(cudaMemsetAsync(E->rdf_acc, 0, (size_t)S * S * E->rdf_nbins * sizeof(unsigned long long), E->stream));
     }
-    rc = prepare_step_state(E, 0);
-    if (rc) return rc;
+    if (one) {
+        CK(cudaMemsetAsync(E->counts, 0, E->ncells_tot * sizeof(int), E->stream));
+        E->step_h = 0;
+    } else {
+        rc = prepare_step_state(E, 0);
+        if (rc) return rc;
+    }
     E->part_off = off;
     if (list_mode) {
         rc = ensure_list(E, list_cap_estimate(E), E->list_wide);
-        if (!rc) rc = resort<R>(E, true);
+        if (!rc) rc = resort<R>(E, true, one);
         if (rc) { E->part_off.clear(); return rc; }
     }
     return RDGPU_OK;
@@ -1818,13 +1853,9 @@ template <class R> int grow_preserving(Engine* E, long long n)
 // the appended ones follow; ids are renumbered 0 .. n-1 in that order.
 template <class R> int apply_edits_impl(Engine* E, const float* ed, long long count)
 {
-    {
-        const int rc = sync_types<R>(E);
-        if (rc) return rc;
-    }
     const long long N = E->npart_tot;
     const int S = E->desc.n_types;
-    std::vector<char> gone(std::max<long long>(N, 1), 0);
+    std::unordered_set<int> gone;
     std::vector<int> del;
     std::vector<double> axyz;
     std::vector<int> atype;
@@ -1836,9 +1867,8 @@ template <class R> int apply_edits_impl(Engine* E, const float* ed, long long co
         const long long index = (long long)fi;
         const int newType = (int)ft;
         if (index != -1) {
-            if (index < 0 || index >= N || gone[index])
+            if (index < 0 || index >= N || !gone.insert((int)index).second)
                 return fail(E, RDGPU_ERR_ARG, "reaction entry " + std::to_string(r) + ": invalid or repeated gpu index");
-            gone[index] = 1;
             del.push_back((int)index);
         }
         if (newType != -1) {
@@ -1911,22 +1941,22 @@ template <class R> int apply_edits_impl(Engine* E, const float* ed, long long co
     E->part_off = {0, N2};
     CK(cudaMemsetAsync(E->sys_of, 0, std::max<long long>(N2, 1) * sizeof(unsigned short), E->stream));
     CK(cudaMemcpyAsync(E->sys_d, E->sys_h.data(), sizeof(SysDev), cudaMemcpyHostToDevice, E->stream));
-    launch_sort<R>(E);
+    const bool one = E->nb_mode == RDGPU_NB_LIST && N2 > 0 && run_in_one(E);
+    if (one) {
+        // the list build below sorts the staged particles itself
+        set_cur(E, E->cur ^ 1);
+        CK(cudaMemsetAsync(E->counts, 0, E->ncells_tot * sizeof(int), E->stream));
+    } else {
+        launch_sort<R>(E);
+    }
     CK(cudaGetLastError());
-    // host copy of the types by id
-    std::vector<int> nt;
-    nt.reserve(N2);
-    for (long long i = 0; i < N; ++i)
-        if (!gone[i]) nt.push_back(E->types_h[i]);
-    for (int t : atype) nt.push_back(t);
-    E->types_h.swap(nt);
-    E->types_h_valid = true;
+    E->types_h_valid = false;     // (downloaded when needed, sync_types)
     // bonds: those of deleted particles go, the rest follow the new ids
     if (!E->bond_pot_h.empty()) {
         std::vector<int> nid(std::max<long long>(N, 1), -1);
         long long c = 0;
         for (long long i = 0; i < N; ++i)
-            if (!gone[i]) nid[i] = (int)c++;
+            if (!gone.count((int)i)) nid[i] = (int)c++;
         std::vector<int> ij, pot;
         for (size_t b = 0; b < E->bond_pot_h.size(); ++b) {
             const int i = nid[E->bond_ij_h[2 * b]], j = nid[E->bond_ij_h[2 * b + 1]];
@@ -1940,8 +1970,10 @@ template <class R> int apply_edits_impl(Engine* E, const float* ed, long long co
         rc = upload_bonds<R>(E);
         if (rc) { E->part_off.clear(); return rc; }
     }
-    rc = reset_counters(E, E->step_h);
-    if (rc) return rc;
+    if (!one) {
+        rc = reset_counters(E, E->step_h);
+        if (rc) return rc;
+    }
     if (E->nb_mode == RDGPU_NB_LIST && N2 > 0) {
         rc = ensure_list(E, list_cap_estimate(E), E->list_wide);
         if (!rc) rc = resort<R>(E, true);

@@ -36,6 +36,9 @@ struct RunOut {
     long long t;    // the next step to compute
 };
 
+constexpr int RUN_REBUILD = 1;
+constexpr int RUN_REBUILD_INPUT = 2;   // the same, unless a.err says that the upload was rejected
+
 template <class R> struct RunArgs {
     Args<R> a;
     ListArgs<R> v;
@@ -47,6 +50,7 @@ template <class R> struct RunArgs {
     long long t0;      // first step
     int nsteps;
     int sel0;          // the buffer that holds its input
+    int rebuild;       // RUN_REBUILD: re-sort and build the lists first
 };
 
 // Threads per block, at most; one block per SM.  Its warps draw the SM's tiles
@@ -430,7 +434,18 @@ __global__ void __launch_bounds__(HOME > 0 ? run_home_block(HOME) : RunShape<R, 
         sh.sorted = 0;
         sh.rankable = sh.own > (int)(blockDim.x >> 5) && sh.own <= RUN_ORDER;
     }
-    while (t < tend) {
+    if (p.rebuild) {
+        err = p.rebuild == RUN_REBUILD_INPUT ? *((volatile const int*)a.err) : 0;
+        if (!err) {
+            alive = run_rebuild<R>(p, sh, sel, 0);
+            err = alive ? sh.err : 0;
+            if (alive && !err) {
+                sel ^= 1;
+                ++builds;
+            }
+        }
+    }
+    while (t < tend && alive && !err) {
         const State<R> cur = sel ? v.b1 : v.b0;
         const State<R> nxt = sel ? v.b0 : v.b1;
         const int after = slot == 2 ? 0 : slot + 1;
