@@ -42,6 +42,10 @@ constexpr int kCheckBlock = 256;
 constexpr int kCheckBlocks = 512;
 // steps of one list_run_kernel launch, at most
 constexpr long long kRunSteps = 1024;
+// downloads up to this size (a block's shared memory without the opt-in) go
+// through the handle's page-locked memory: the kernel writes them there, which
+// spares two copies and their queueing
+constexpr size_t kFrameBytes = 48 * 1024;
 constexpr const char* kBadInput = "particle type out of range, non-finite coordinate, or a coordinate more than 64 box "
                                   "lengths outside the box";
 }  // namespace
@@ -54,6 +58,7 @@ struct Pinned {
     long long step;
     ListCtl ctl;
     RunOut run;
+    alignas(16) char frame[kFrameBytes];   // a small download, written by emit_small_kernel
 };
 
 // the opaque handle type of the C ABI
@@ -1986,6 +1991,17 @@ template <class R, class Out> int get_particles_impl(Engine* E, Out* xyz, int* t
 {
     const long long N = E->npart_tot;
     if (N == 0) return RDGPU_OK;
+    const size_t xb = (size_t)N * 3 * sizeof(Out), tb = (size_t)N * sizeof(int);
+    if (xb + tb <= kFrameBytes) {
+        char* f = E->pinned->frame;
+        const size_t smem = (xb + tb + 15) & ~(size_t)15;
+        emit_small_kernel<R, Out><<<1, 1024, smem, E->stream>>>(E->sys_d, E->sys_of, (int)N, cur_state<R>(E), (int4*)f);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(E->stream));
+        if (xyz) memcpy(xyz, f, xb);
+        if (types) memcpy(types, f + xb, tb);
+        return RDGPU_OK;
+    }
     emit_kernel<R, Out><<<grid_for(N), 256, 0, E->stream>>>(E->sys_d, E->sys_of, N, cur_state<R>(E), (Out*)E->vec_d,
                                                             E->ityp_d);
     CK(cudaGetLastError());

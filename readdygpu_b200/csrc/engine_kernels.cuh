@@ -965,31 +965,52 @@ __global__ void edit_append_kernel(const SysDev* __restrict__ sys, long long bas
                       x0n, err);
 }
 
-// sorted arrays -> absolute coordinates (FP64, or rounded to FP32) and types
-// by global index
+// particle i of the sorted arrays to absolute coordinates (FP64, or rounded to
+// FP32) and type by global index
+template <class R, class Out>
+__device__ __forceinline__ void emit_one(const SysDev& s, long long i, const State<R>& cur, Out* xyz, int* types)
+{
+    if constexpr (sizeof(R) == 4) {
+        const float4 p = cur.pos[i], c = cur.aux[i];
+        const long long g = s.part_base + __float_as_int(c.w);
+        xyz[3 * g + 0] = (Out)__dadd_rn(__dsub_rn((double)p.x, (double)c.x), s.lo[0]);
+        xyz[3 * g + 1] = (Out)__dadd_rn(__dsub_rn((double)p.y, (double)c.y), s.lo[1]);
+        xyz[3 * g + 2] = (Out)__dadd_rn(__dsub_rn((double)p.z, (double)c.z), s.lo[2]);
+        types[g] = __float_as_int(p.w) & 0xff;
+    } else {
+        const Rec64 r = cur.rec[i];
+        const long long g = s.part_base + r.id;
+        xyz[3 * g + 0] = (Out)__dadd_rn(r.x, s.lo[0]);
+        xyz[3 * g + 1] = (Out)__dadd_rn(r.y, s.lo[1]);
+        xyz[3 * g + 2] = (Out)__dadd_rn(r.z, s.lo[2]);
+        types[g] = r.w & 0xff;
+    }
+}
+
 template <class R, class Out>
 __global__ void emit_kernel(const SysDev* __restrict__ sys, const unsigned short* __restrict__ sys_of, long long ntot,
                             State<R> cur, Out* __restrict__ xyz, int* __restrict__ types)
 {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ntot;
-         i += (long long)gridDim.x * blockDim.x) {
-        const SysDev& s = sys[sys_of[i]];
-        if constexpr (sizeof(R) == 4) {
-            const float4 p = cur.pos[i], c = cur.aux[i];
-            const long long g = s.part_base + __float_as_int(c.w);
-            xyz[3 * g + 0] = (Out)__dadd_rn(__dsub_rn((double)p.x, (double)c.x), s.lo[0]);
-            xyz[3 * g + 1] = (Out)__dadd_rn(__dsub_rn((double)p.y, (double)c.y), s.lo[1]);
-            xyz[3 * g + 2] = (Out)__dadd_rn(__dsub_rn((double)p.z, (double)c.z), s.lo[2]);
-            types[g] = __float_as_int(p.w) & 0xff;
-        } else {
-            const Rec64 r = cur.rec[i];
-            const long long g = s.part_base + r.id;
-            xyz[3 * g + 0] = (Out)__dadd_rn(r.x, s.lo[0]);
-            xyz[3 * g + 1] = (Out)__dadd_rn(r.y, s.lo[1]);
-            xyz[3 * g + 2] = (Out)__dadd_rn(r.z, s.lo[2]);
-            types[g] = r.w & 0xff;
-        }
-    }
+         i += (long long)gridDim.x * blockDim.x)
+        emit_one<R, Out>(sys[sys_of[i]], i, cur, xyz, types);
+}
+
+// The same for a small handle, one block: ordered in shared memory (coordinates,
+// then types), then to page-locked host memory in whole words.  (Scattered
+// writes straight to the host cost 9 us per 1,000 particles.)
+template <class R, class Out>
+__global__ void __launch_bounds__(1024) emit_small_kernel(const SysDev* __restrict__ sys,
+                                                          const unsigned short* __restrict__ sys_of, int ntot,
+                                                          State<R> cur, int4* __restrict__ host)
+{
+    extern __shared__ __align__(16) char emit_out[];
+    Out* xyz = reinterpret_cast<Out*>(emit_out);
+    int* types = reinterpret_cast<int*>(xyz + 3 * ntot);
+    for (int i = threadIdx.x; i < ntot; i += blockDim.x) emit_one<R, Out>(sys[sys_of[i]], i, cur, xyz, types);
+    __syncthreads();
+    const int words = (int)((ntot * (3 * sizeof(Out) + sizeof(int)) + 15) / 16);
+    for (int k = threadIdx.x; k < words; k += blockDim.x) host[k] = reinterpret_cast<const int4*>(emit_out)[k];
 }
 
 // ---------------------------------------------------------------------------

@@ -224,3 +224,17 @@ def test_run_tiles_in_the_order_of_their_cost(prec):
     xc, xr, nb = both(prec, w.system, w.xyz, w.types, [40, 1, 19])
     assert nb > 1
     same(prec, xc, xr)
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+@pytest.mark.parametrize("out", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [1, 1755, 1756, 3072, 3073])
+def test_download_sizes(prec, out, n):
+    """Downloads up to 48 KB (1,755 FP64 or 3,072 FP32 frames) and larger ones
+    return the particles in their order, in either coordinate type."""
+    sys_, xyz, types = plain(n)
+    xyz = xyz.astype(np.float32)
+    with Engine(sys_, precision=prec) as e:
+        e.set_particles(xyz, types)
+        x, t = e.get_particles(np.empty((n, 3), out), np.empty(n, np.int32))
+    assert np.array_equal(x, xyz.astype(out)) and np.array_equal(t, types)
