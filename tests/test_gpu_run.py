@@ -238,3 +238,82 @@ def test_download_sizes(prec, out, n):
         e.set_particles(xyz, types)
         x, t = e.get_particles(np.empty((n, 3), out), np.empty(n, np.int32))
     assert np.array_equal(x, xyz.astype(out)) and np.array_equal(t, types)
+
+
+def test_run_wide_entries():
+    """32-bit list entries in the run kernel."""
+    sys_, xyz, types, width = slab()
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision="f32c", seed=3, neighbour_mode=mode) as e:
+            e.set_particles(xyz, types)
+            e.autotune()
+            e.step(40)
+            m = e.metrics()
+            out.append(e.get_particles()[0])
+    assert m["neighbour_mode"] == "list" and m["list_entry_bytes"] == width
+    same("f32c", out[0], out[1])
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+def test_run_with_bonds_edits_and_uploads(prec):
+    """Bonded chains, reaction edits, a rejected upload and a new upload on a
+    handle whose steps and list builds run in one launch: the cell walk's
+    positions throughout."""
+    sys_, xyz, types = plain(3000)
+    chain = [PairPotential(A.P2_HARMONIC, [], 5.0, "spring", r0=3.0)]
+    ij = np.array([[k, k + 1] for k in range(0, 600) if k % 6 != 5])
+    gone = [[k, -1, 0, 0, 0, k] for k in (0, 17, 599, 2999)]
+    born = [[0, 1, 5.0 + k, 6.0, 7.0, -1] for k in range(3)]
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision=prec, seed=6, neighbour_mode=mode) as e:
+            e.set_particles(xyz, types)
+            e.autotune()
+            e.set_bonds(ij, np.zeros(len(ij), np.int32), chain)
+            got = []
+            e.step(60)
+            got.append(e.get_particles()[0])
+            e.apply_edits(gone + born)
+            e.step(60)
+            got.append(e.get_particles()[0])
+            got.append(e.forces()[0])
+            for bad_x, bad_t in ((np.nan, 0), (1e6, 0), (1.0, 7)):
+                bx, bt = xyz.copy(), types.copy()
+                bx[5, 1], bt[5] = bad_x, bad_t
+                with pytest.raises(RdgpuError) as err:
+                    e.set_particles(bx, bt)
+                assert err.value.code == -1
+            e.set_particles(xyz[::-1], types[::-1])
+            e.step(30)
+            got.append(e.get_particles()[0])
+            assert e.metrics()["step"] == 30
+        out.append(got)
+    for a, b in zip(*out):
+        same(prec, a, b)
+
+
+def test_two_handles_in_two_threads():
+    """Two handles too large to be resident together, stepped at the same time
+    from two threads, go their own way unchanged."""
+    import threading
+    sys_, xyz, types = plain(160_000)
+    alone, together = {}, {}
+
+    def go(seed, out):
+        with Engine(sys_, precision="f32c", seed=seed) as e:
+            e.set_particles(xyz, types)
+            e.autotune()
+            for _ in range(6):
+                e.step(50)
+            out[seed] = e.get_particles()[0]
+
+    for seed in (1, 2):
+        go(seed, alone)
+    ts = [threading.Thread(target=go, args=(seed, together)) for seed in (1, 2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for seed in (1, 2):
+        assert np.array_equal(alone[seed], together[seed])
