@@ -388,6 +388,7 @@ void free_particles(Engine* E)
     for (int b = 0; b < 2; ++b) { dfree(E->bufA[b]); dfree(E->bufB[b]); }
     dfree(E->tcell); dfree(E->tslot);
     dfree(E->nbr); dfree(E->head); dfree(E->hot);
+    E->list_valid = false;
     E->list_stride = 0;
     E->list_cap = 0;
     dfree(E->sys_of); dfree(E->x0_d); dfree(E->vec_d); dfree(E->val_d); dfree(E->ityp_d); dfree(E->u64_d);
@@ -1007,14 +1008,18 @@ template <class R> int run_steps(Engine* E, int n, int rebuild = 0)
 }
 
 // Re-sorts the current state (the input of step step_h) by cell into the
-// other buffer and, with_list, builds the pair lists; an overflowing build
-// grows the lists and is redone.
+// other buffer and, with_list, builds the pair lists (in storage made here if
+// there is none); an overflowing build grows the lists and is redone.
 // check_input: the state comes from an upload that the kernels may have
 // rejected (RDGPU_ERR_ARG then).
 template <class R> int resort(Engine* E, bool with_list, bool check_input = false)
 {
     if (E->npart_tot == 0) return RDGPU_OK;
     E->list_valid = false;
+    if (with_list) {
+        const int rc = ensure_list(E, list_cap_estimate(E), E->list_wide);
+        if (rc) return rc;
+    }
     if (with_list && run_in_one(E)) {
         // all of it in one launch and one wait (chain of launches: six, and
         // three waits; 20,000 particles FP64 171 -> 99 us per upload)
@@ -1089,9 +1094,7 @@ template <class R> int enter_list(Engine* E, double skin)
             CK(cudaMemcpy(E->rl2_d, t.data(), MAXT * MAXT * rs, cudaMemcpyHostToDevice));
         }
     }
-    if (E->part_off.empty() || E->npart_tot == 0) return RDGPU_OK;
-    int rc = ensure_list(E, list_cap_estimate(E), E->list_wide);
-    if (rc) return rc;
+    if (E->part_off.empty()) return RDGPU_OK;
     return resort<R>(E, true);
 }
 
@@ -1247,9 +1250,7 @@ template <class R> int do_steps_list(Engine* E, long long nsteps, const double* 
 // that had grown the buffers, or a failed re-sort)
 template <class R> int need_lists(Engine* E)
 {
-    if (E->nb_mode != RDGPU_NB_LIST || E->list_valid) return RDGPU_OK;
-    const int rc = ensure_list(E, list_cap_estimate(E), E->list_wide);
-    return rc ? rc : resort<R>(E, true);
+    return E->nb_mode == RDGPU_NB_LIST && !E->list_valid ? resort<R>(E, true) : RDGPU_OK;
 }
 
 template <class R> int do_steps_mode(Engine* E, long long nsteps, const double* noise_d)
@@ -1817,15 +1818,16 @@ template <class R, class In> int set_particles_impl(Engine* E, const long long* 
     }
     E->part_off = off;
     if (list_mode) {
-        rc = ensure_list(E, list_cap_estimate(E), E->list_wide);
-        if (!rc) rc = resort<R>(E, true, one);
+        rc = resort<R>(E, true, one);
         if (rc) { E->part_off.clear(); return rc; }
     }
     return RDGPU_OK;
 }
 
-// grows the per-particle buffers to hold n particles, keeping the current
-// state and the MSD origins of the first npart_tot particles
+// grows the per-particle buffers to hold n particles, keeping all that steps
+// and evaluations of the first npart_tot particles read: the sorted state, its
+// systems, the sorted index of every id (bonds) and the MSD origins (a
+// rejected edit goes on from them; the pair lists, freed here, are built anew)
 template <class R> int grow_preserving(Engine* E, long long n)
 {
     if (n <= E->cap_particles) return RDGPU_OK;
@@ -1834,9 +1836,13 @@ template <class R> int grow_preserving(Engine* E, long long n)
     void* keepA = E->bufA[E->cur];
     void* keepB = E->bufB[E->cur];
     double* keepX0 = E->x0_d;
+    unsigned short* keepSys = E->sys_of;
+    int* keepInv = E->inv;
     E->bufA[E->cur] = nullptr;
     E->bufB[E->cur] = nullptr;
     E->x0_d = nullptr;
+    E->sys_of = nullptr;
+    E->inv = nullptr;
     int rc = ensure_particle_buffers(E, n);    // new buffers, current state in buffer 0
     if (rc == RDGPU_OK && nold > 0) {
         cudaError_t e = cudaMemcpyAsync(E->bufA[0], keepA, nold * recA, cudaMemcpyDeviceToDevice, E->stream);
@@ -1844,12 +1850,18 @@ template <class R> int grow_preserving(Engine* E, long long n)
             e = cudaMemcpyAsync(E->bufB[0], keepB, nold * 16, cudaMemcpyDeviceToDevice, E->stream);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(E->x0_d, keepX0, nold * 3 * sizeof(double), cudaMemcpyDeviceToDevice, E->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(E->sys_of, keepSys, nold * sizeof(*keepSys), cudaMemcpyDeviceToDevice, E->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(E->inv, keepInv, nold * sizeof(*keepInv), cudaMemcpyDeviceToDevice, E->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(E->stream);
         if (e != cudaSuccess) rc = fail(E, RDGPU_ERR_CUDA, std::string("buffer growth: ") + cudaGetErrorString(e));
     }
     cudaFree(keepA);
     if (keepB) cudaFree(keepB);
     cudaFree(keepX0);
+    cudaFree(keepSys);
+    cudaFree(keepInv);
     return rc;
 }
 
@@ -1889,7 +1901,6 @@ template <class R> int apply_edits_impl(Engine* E, const float* ed, long long co
     if (nd == 0 && na == 0) return RDGPU_OK;
     const long long nkeep = N - nd, N2 = nkeep + na;
     if (N2 > 0x7fffffff) return fail(E, RDGPU_ERR_ARG, "at most 2^31-1 particles per handle");
-    E->list_valid = false;
     int rc = grow_preserving<R>(E, N2);
     if (rc) { E->part_off.clear(); return rc; }
     drop_graphs(E);   // launch shapes depend on the particle count
@@ -1940,6 +1951,7 @@ template <class R> int apply_edits_impl(Engine* E, const float* ed, long long co
         return fail(E, RDGPU_ERR_ARG, "appended particle with a non-finite coordinate or far outside the box");
     }
     // the new MSD origins and particle count, then the counting sort staging -> current
+    E->list_valid = false;
     if (N2 > 0) CK(cudaMemcpyAsync(E->x0_d, E->vec_d, N2 * 3 * sizeof(double), cudaMemcpyDeviceToDevice, E->stream));
     E->npart_tot = N2;
     E->sys_h[0].npart = (int)N2;
@@ -1979,9 +1991,8 @@ template <class R> int apply_edits_impl(Engine* E, const float* ed, long long co
         rc = reset_counters(E, E->step_h);
         if (rc) return rc;
     }
-    if (E->nb_mode == RDGPU_NB_LIST && N2 > 0) {
-        rc = ensure_list(E, list_cap_estimate(E), E->list_wide);
-        if (!rc) rc = resort<R>(E, true);
+    if (E->nb_mode == RDGPU_NB_LIST) {
+        rc = resort<R>(E, true);
         if (rc) { E->part_off.clear(); return rc; }
     }
     return RDGPU_OK;
@@ -2026,10 +2037,11 @@ template <class R> int sync_types(Engine* E)
 }
 
 // a walk over the cells in pair-list mode: re-sort first (the particles have
-// moved since the last build)
+// moved since the last build).  Valid lists are built for the new order at
+// once; missing ones, which the walk can do without, by the next step.
 template <class R> int fresh_cells(Engine* E)
 {
-    return E->nb_mode == RDGPU_NB_LIST ? resort<R>(E, true) : RDGPU_OK;
+    return E->nb_mode == RDGPU_NB_LIST ? resort<R>(E, E->list_valid) : RDGPU_OK;
 }
 
 // forces and energies (MODE 1) or neighbour digest (MODE 2) of the current

@@ -1,0 +1,69 @@
+"""Handles in pair-list mode whose lists are gone: after a rejected edit that had
+grown the buffers, steps, forces, energies, neighbour sets and RDF frames are
+those of a handle that never saw the edit."""
+import numpy as np
+import pytest
+
+from readdygpu_b200 import RdgpuError, _abi as A
+from readdygpu_b200.system import PairPotential
+
+from .test_gpu_pairlist import same
+from .test_gpu_parity import Engine
+from .test_gpu_run import plain
+
+pytestmark = pytest.mark.gpu
+
+
+def reject(e, n, born):
+    """An edit that deletes one particle and appends `born`, the last of them off the chart."""
+    rows = [[0, -1, 0, 0, 0, 7]] + [[1, k % 2, 1.0 + 0.1 * k, 2.0, 3.0, -1] for k in range(born)]
+    rows[-1][3] = np.nan
+    with pytest.raises(RdgpuError) as err:
+        e.apply_edits(rows)
+    assert err.value.code == -1 and e.n == n
+
+
+def observe(e):
+    cnt, h = e.neighbor_digest()
+    F, en = e.forces()
+    return [e.get_particles()[0], F, np.array([en, e.metrics()["energy"]]), cnt, h, e.rdf(40, 18.0, False)[0]]
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+@pytest.mark.parametrize("mode", ["cells", "list", "auto"])
+@pytest.mark.parametrize("bonds", [False, True])
+@pytest.mark.parametrize("born", [3, 300])
+def test_rejected_edit_changes_nothing(prec, mode, bonds, born):
+    """400 particles have room for 100 more: 3 appended ones fit, 300 grow the
+    buffers before their coordinates are looked at."""
+    sys_, xyz, types = plain(400)
+    ij = np.array([[k, k + 1] for k in range(0, 60) if k % 6 != 5])
+    chain = [PairPotential(A.P2_HARMONIC, [], 5.0, "spring", r0=3.0)]
+    out = []
+    for m, rejecting in (("cells", False), (mode, True)):
+        with Engine(sys_, precision=prec, seed=9, neighbour_mode=m, skin=0.8 if m == "list" else 0.0) as e:
+            e.set_particles(xyz, types)
+            if m == "auto":
+                e.autotune()
+                assert e.metrics()["neighbour_mode"] == "list"
+            if bonds:
+                e.set_bonds(ij, np.zeros(len(ij), np.int32), chain)
+            e.step(25)
+            got = []
+            if rejecting:
+                reject(e, 400, born)
+            got += observe(e)           # evaluated before the next step
+            e.step(30)
+            got += observe(e)
+            if rejecting:
+                reject(e, 400, 2 * born)
+            e.step(30)                  # stepped before any evaluation
+            got += observe(e)
+            out.append(got)
+    for a, b in zip(*out):
+        if a.dtype.kind in "iu":
+            assert np.array_equal(a, b)
+        elif len(a) == 2:               # energies: FP32 or FP64 sums over the cells, FP64 over the lists
+            assert np.abs(a - b).max() <= (1e-5 if prec == "f32c" else 1e-10) * np.abs(a).max()
+        else:
+            same(prec, a, b)
