@@ -195,10 +195,13 @@ using Engine = rdgpu_engine;
 
 template <class R> int sync_types(Engine* E);
 
+// a failed call is reported once: it leaves its code for cudaGetLastError() too,
+// where the check after the next launch would take it for that launch's
 #define CK(call)                                                                   \
     do {                                                                           \
         cudaError_t e_ = (call);                                                   \
         if (e_ != cudaSuccess) {                                                   \
+            cudaGetLastError();                                                    \
             E->last_error = std::string(#call) + ": " + cudaGetErrorString(e_);   \
             return (e_ == cudaErrorMemoryAllocation) ? RDGPU_ERR_NOMEM : RDGPU_ERR_CUDA; \
         }                                                                          \
@@ -640,6 +643,9 @@ int configure_cells(Engine* E, double cut, std::string& why)
         if (cudaMalloc(&E->start, (cb + 1) * sizeof(int)) != cudaSuccess ||
             cudaMalloc(&E->counts, std::max<long long>(cb, 1) * sizeof(int)) != cudaSuccess ||
             cudaMalloc(&E->tile_sum, std::max(ntiles, 1) * sizeof(int)) != cudaSuccess) {
+            cudaGetLastError();
+            dfree(E->start); dfree(E->counts); dfree(E->tile_sum);
+            E->cell_cut = -1.0;    // no grid
             why = "device allocation failed";
             return RDGPU_ERR_NOMEM;
         }
@@ -1904,7 +1910,7 @@ template <class R> int apply_edits_impl(Engine* E, const float* ed, long long co
     int rc = grow_preserving<R>(E, N2);
     if (rc) { E->part_off.clear(); return rc; }
     drop_graphs(E);   // launch shapes depend on the particle count
-    auto bad = [&](const char* what) { E->part_off.clear(); return fail(E, RDGPU_ERR_CUDA, what); };
+    auto bad = [&](const char* what) { cudaGetLastError(); E->part_off.clear(); return fail(E, RDGPU_ERR_CUDA, what); };
     // the frame's edits on the device: appended coordinates, types, deleted indices
     const size_t need = (size_t)na * 3 * sizeof(double) + (size_t)(na + nd) * sizeof(int);
     if (need > E->ed_buf_bytes) {
@@ -2372,6 +2378,7 @@ int create_impl(const rdgpu_system_desc* desc, int nsys, const rdgpu_box* boxes,
     E->nb_req = o.neighbour_mode;
     E->skin_req = o.skin;
     auto bail = [&](int code, const std::string& msg) {
+        cudaGetLastError();
         g_create_error = msg;
         rdgpu_destroy(E);
         return code;

@@ -1,6 +1,7 @@
-"""Handles in pair-list mode whose lists are gone: after a rejected edit that had
+"""Handles in pair-list mode whose lists are gone.  After a rejected edit that had
 grown the buffers, steps, forces, energies, neighbour sets and RDF frames are
-those of a handle that never saw the edit."""
+those of a handle that never saw the edit.  When the lists outgrow the device
+memory, the call that needs them says so and the rest goes on."""
 import numpy as np
 import pytest
 
@@ -67,3 +68,27 @@ def test_rejected_edit_changes_nothing(prec, mode, bonds, born):
             assert np.abs(a - b).max() <= (1e-5 if prec == "f32c" else 1e-10) * np.abs(a).max()
         else:
             same(prec, a, b)
+
+
+def clot(n=1_600_000, m=25_000):
+    """m of n particles drawn into a cube of edge 1: lists that hold theirs would
+    take 200 GB (16-bit entries) or more.  Next to no force, so that the clot stays."""
+    sys_, xyz, types = plain(n)
+    sys_.pair[0].k = 1e-3
+    packed = xyz.copy()
+    packed[:m] = 0.5 * sys_.hi[0] + np.random.default_rng(1).uniform(0, 1.0, (m, 3))
+    return sys_, xyz, packed, types
+
+
+def test_untuned_handle_whose_lists_do_not_fit_keeps_the_cell_walk():
+    sys_, _, packed, types = clot()
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision="f32c", seed=2, neighbour_mode=mode) as e:
+            e.set_particles(packed, types)
+            e.step(40)
+            e.step(3)
+            m = e.metrics()
+            out.append(e.get_particles()[0])
+    assert m["neighbour_mode"] == "cells" and m["step"] == 43
+    assert np.array_equal(out[0], out[1])
