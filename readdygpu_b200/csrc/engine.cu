@@ -637,6 +637,7 @@ int configure_cells(Engine* E, double cut, std::string& why)
     }
     if (cb >= 0x7fffffffLL) { why = "too many cells in the batch"; return RDGPU_ERR_ARG; }
     drop_graphs(E);
+    E->list_valid = false;     // the lists are checked on the grid they were built on
     const int ntiles = (int)((cb + SCAN_TILE - 1) / SCAN_TILE);
     if (cb > E->ncells_tot || !E->start) {
         dfree(E->start); dfree(E->counts); dfree(E->tile_sum);
@@ -747,6 +748,7 @@ int ensure_list(Engine* E, int cap, bool wide)
     cap = std::min((std::max(std::max(cap, E->list_cap), 8) + 7) & ~7, 65528);
     drop_graph_map(E->lgraphs);
     dfree(E->nbr); dfree(E->head); dfree(E->hot);
+    E->list_valid = false;
     E->list_cap = 0;
     E->list_stride = 0;
     const long long groups = wide ? cap / 4 : cap / 8;
@@ -773,6 +775,8 @@ int list_regrow_cap(Engine* E)
 // than the capacity; EF_LISTWIDE: an offset beyond 16 bits)
 int ensure_list_after(Engine* E, int ef)
 {
+    // taken note of: the scans of other calls (an RDF frame) stop at a set flag
+    CK(cudaMemsetAsync(E->err, 0, sizeof(int), E->stream));
     const int cap = (ef & EF_LISTOVF) ? list_regrow_cap(E) : E->list_cap;
     return ensure_list(E, cap, E->list_wide || (ef & EF_LISTWIDE) != 0);
 }
@@ -1253,7 +1257,7 @@ template <class R> int do_steps_list(Engine* E, long long nsteps, const double* 
 }
 
 // pair-list mode: lists of the current state (missing after a rejected edit
-// that had grown the buffers, or a failed re-sort)
+// that had grown the buffers, a failed re-sort, or lists that outgrew the memory)
 template <class R> int need_lists(Engine* E)
 {
     return E->nb_mode == RDGPU_NB_LIST && !E->list_valid ? resort<R>(E, true) : RDGPU_OK;

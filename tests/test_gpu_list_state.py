@@ -92,3 +92,48 @@ def test_untuned_handle_whose_lists_do_not_fit_keeps_the_cell_walk():
             out.append(e.get_particles()[0])
     assert m["neighbour_mode"] == "cells" and m["step"] == 43
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("mode", ["list", "auto"])
+def test_lists_that_outgrow_the_memory_in_a_step(mode):
+    """The step that draws the particles together stands and its lists are
+    refused; the state can be read and evaluated, steps are refused as long as
+    it lasts, and the next upload steps on."""
+    sys_, xyz, packed, types = clot()
+    n = len(xyz)
+    b = np.sqrt(2.0 * np.array([t.D for t in sys_.types])[types] * sys_.dt)[:, None]
+    with Engine(sys_, precision="f64", seed=2, neighbour_mode=mode, skin=1.0 if mode == "list" else 0.0) as e:
+        e.set_particles(xyz, types)
+        if mode == "auto":
+            e.autotune()
+        assert e.metrics()["neighbour_mode"] == "list"
+        with pytest.raises(RdgpuError) as err:
+            e.step_with_noise((packed - xyz) / b)
+        assert err.value.code == -6
+        m = e.metrics()
+        assert m["step"] == 1 and m["neighbour_mode"] == "list"
+        x, t = e.get_particles()
+        assert np.abs(x - packed).max() < 1e-3
+        F, en = e.forces()
+        cnt, h = e.neighbor_digest()
+        with Engine(sys_, precision="f64", neighbour_mode="cells") as c:
+            c.set_particles(x, t)
+            Fc, enc = c.forces()
+            cntc, hc = c.neighbor_digest()
+            gc = c.rdf(20, 6.0, False)[0]
+        assert np.array_equal(cnt, cntc) and np.array_equal(h, hc)
+        assert np.linalg.norm(F - Fc) <= 1e-11 * np.linalg.norm(Fc)
+        assert abs(en - enc) <= 1e-10 * abs(enc) and m["energy"] == pytest.approx(en, rel=1e-10)
+        for _ in range(2):
+            with pytest.raises(RdgpuError) as err:
+                e.step(1)
+            assert err.value.code == -6
+        assert np.array_equal(e.rdf(20, 6.0, False)[0], gc)
+        assert e.forces()[1] == pytest.approx(enc, rel=1e-10)
+        e.set_particles(xyz, types)
+        e.step(30)
+        y, _ = e.get_particles()
+    with Engine(sys_, precision="f64", seed=2, neighbour_mode="cells") as c:
+        c.set_particles(xyz, types)
+        c.step(30)
+        same("f64", c.get_particles()[0], y)
