@@ -1037,7 +1037,11 @@ template <class R> int resort(Engine* E, bool with_list, bool check_input = fals
             int rc = run_steps<R>(E, 0, check_input ? RUN_REBUILD_INPUT : RUN_REBUILD);
             if (rc) return rc;
             const RunOut o = *E->run_out;
-            if (o.dead) return fail(E, RDGPU_ERR_CUDA, "a grid barrier of the list build timed out");
+            if (o.dead) {
+                // the cells may be half counted: nothing runs on them before the next upload clears them
+                E->part_off.clear();
+                return fail(E, RDGPU_ERR_CUDA, "a grid barrier of the list build timed out");
+            }
             if (o.err & EF_BADINPUT) return fail(E, RDGPU_ERR_ARG, kBadInput);
             if (o.err == 0) {
                 set_cur(E, o.sel);
@@ -1319,13 +1323,19 @@ template <class R> int tune(Engine* E)
         if (rc) break;
         // a trial that fails (the dynamics itself, e.g. a particle leaving the
         // box) disqualifies the candidate; the real run reports the failure
-        if (do_steps_mode<R>(E, E->graph_steps, nullptr) != RDGPU_OK) continue;
+        if (do_steps_mode<R>(E, E->graph_steps, nullptr) != RDGPU_OK) {
+            if (E->part_off.empty()) { rc = RDGPU_ERR_CUDA; break; }   // the state is gone
+            continue;
+        }
         // three graphs: several rebuild intervals of the larger skins
         cudaEventRecord(e0, E->stream);
         const int trial = do_steps_mode<R>(E, 3LL * E->graph_steps, nullptr);
         cudaEventRecord(e1, E->stream);
         cudaEventSynchronize(e1);
-        if (trial != RDGPU_OK) continue;
+        if (trial != RDGPU_OK) {
+            if (E->part_off.empty()) { rc = RDGPU_ERR_CUDA; break; }
+            continue;
+        }
         float ms = 0.f;
         cudaEventElapsedTime(&ms, e0, e1);
         if (ms < best_ms) { best_ms = ms; best_skin = skins[c]; }
