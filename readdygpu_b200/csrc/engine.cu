@@ -164,6 +164,7 @@ struct rdgpu_engine {
     int* run_tsum = nullptr;             // its scan's tile sums
     long long run_tsum_n = 0;
     int sm_count = 0;
+    const void* run_fn = nullptr;        // the variant of list_run_kernel that the last launch took
     ListCtl* ctl = nullptr;
     ListCtl* pinned_ctl = nullptr;
     int nbuild_h = 0;
@@ -939,11 +940,22 @@ int read_back(Engine* E)
     return RDGPU_OK;
 }
 
-template <class R> int launch_run_as(Engine* E, RunArgs<R>& p, const void* f, int block, int grid, bool home)
+// most: the largest block of f.  The limit on a kernel's dynamic shared memory
+// belongs to the kernel, which all handles and threads of a process share, so
+// every handle sets the same one, the most that any launch of f takes, before
+// its first launch of f (a limit of this launch's own size could be lowered by
+// another thread before the launch).
+template <class R>
+int launch_run_as(Engine* E, RunArgs<R>& p, const void* f, int block, int most, int grid, bool home)
 {
     void* args[] = {&p};
-    const size_t dyn = run_dyn_bytes<R>(block) + (home && !E->hrep ? run_term_bytes<R>(E->desc.n_types) : 0);
-    CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    const bool terms = home && !E->hrep;
+    const size_t dyn = run_dyn_bytes<R>(block) + (terms ? run_term_bytes<R>(E->desc.n_types) : 0);
+    if (E->run_fn != f) {
+        const size_t limit = run_dyn_bytes<R>(most) + (terms ? run_term_bytes<R>(MAXT) : 0);
+        CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+        E->run_fn = f;
+    }
     CK(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(block), args, dyn, E->stream));
     ++E->launches;
     return RDGPU_OK;
@@ -964,19 +976,19 @@ template <class R, bool HREP, bool ALLPER, bool NARROW> int launch_run(Engine* E
     if constexpr (NARROW) {
         if (per_sm <= RUN_HOME_FEW)
             return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_HOME_FEW>,
-                                 32 * ((int)per_sm + 4), grid, true);
+                                 32 * ((int)per_sm + 4), run_home_block(RUN_HOME_FEW), grid, true);
         if (per_sm <= RUN_HOME_MANY)
             return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_HOME_MANY>,
-                                 32 * ((int)per_sm + 3), grid, true);
+                                 32 * ((int)per_sm + 3), run_home_block(RUN_HOME_MANY), grid, true);
     }
     constexpr int most = RunShape<R, HREP, ALLPER>::BLOCK;
     const int block = 32 * (int)std::max<long long>(4, std::min<long long>(most / 32, per_sm));
     if constexpr (NARROW && !HREP) {
         if (per_sm > most / 32)
-            return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_RANK>, block, grid, false);
+            return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, true, RUN_RANK>, block, most, grid,
+                                 false);
     }
-    return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, NARROW, 0>, block, grid,
-                         false);
+    return launch_run_as(E, p, (const void*)list_run_kernel<R, HREP, ALLPER, NARROW, 0>, block, most, grid, false);
 }
 
 template <class R, bool NARROW> int launch_run_w(Engine* E, RunArgs<R>& p, bool allper)
@@ -2199,7 +2211,8 @@ template <class R> int rdf_tiled(Engine* E, int nbins, double rmax)
         nc += m;
     }
     if (nc >= (1LL << 27)) return RDGPU_OK_CONTINUE;
-    if ((size_t)(nbins + 1) * sizeof(float2) > 32 * 1024) return RDGPU_OK_CONTINUE;
+    constexpr size_t most = 32 * 1024;      // dynamic shared memory of rdf_rows_kernel
+    if ((size_t)(nbins + 1) * sizeof(float2) > most) return RDGPU_OK_CONTINUE;
     const long long N = E->npart_tot;
     const size_t recsz = sizeof(RdfRec<R>);
     if (E->rdf_grid_n < E->nsys) {
@@ -2249,15 +2262,15 @@ template <class R> int rdf_tiled(Engine* E, int nbins, double rmax)
                               (1.0 + 1e-3));
     // dynamic shared memory: the edge pairs, then the block's histogram
     const size_t epairs = (size_t)(nbins + 1) * sizeof(float2);
-    const int use_smem = epairs + (size_t)H * 4 <= 32 * 1024 ? 1 : 0;
+    const int use_smem = epairs + (size_t)H * 4 <= most ? 1 : 0;
     const size_t smem = epairs + (use_smem ? (size_t)H * 4 : 0);
     const int grid = (int)std::min<long long>((nc + RDR_WARPS - 1) / RDR_WARPS, 148LL * 8);
     const double w = rmax / (double)nbins;
     // the warps' queues take about 40 KB of static shared memory, so the
-    // dynamic part (up to 32 KB) needs the opt-in above 48 KB per block
+    // dynamic part (up to 32 KB) needs the opt-in above 48 KB per block; always
+    // the same limit, since other threads launch the same kernel
     auto go = [&](auto kernel) {
-        if (smem > 8 * 1024)
-            CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (smem > 8 * 1024) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
         kernel<<<grid, RDR_WARPS * 32, smem, E->stream>>>(E->rdf_grid_d, E->nsys, nc, E->rdf_start, rec, S, nbins,
                                                          E->rdf_e2, w, r2pre, dlt, E->rdf_tmp);
         return RDGPU_OK;
