@@ -711,7 +711,15 @@ template <class R> ListArgs<R> make_list_args(Engine* E, bool with_list)
     // within dq = 2 bins per axis (head_disp2), so it compares the estimate
     // with th - sqrt(3) dq and 2 th - sqrt(3) dq.
     v.rl2t = (const R*)E->rl2_d;
-    const double rl = E->max_rc + E->skin;
+    // A build looks into the cells that may hold a particle within the list
+    // radius, by their distance from the particle along each axis.  That is
+    // rounded by up to 8 x 2^-24 (FP32) of the edge, and not in the same way
+    // seen from the partner.  Twice that on top of the radius keeps every pair
+    // that the distance test (the same from both sides) accepts within reach of
+    // both; with 1e-4 of the squared radius alone, pairs at the list radius were
+    // listed from one side only beyond edges of about 5,500 nm.
+    const double rl = E->max_rc + E->skin +
+                      std::sqrt(3.0) * 16.0 * largest_edge(E) * std::ldexp(1.0, sizeof(R) == 4 ? -24 : -53);
     v.rl2max = (R)(rl * rl * (1.0 + 1e-6));
     const double th = list_threshold(E, E->skin);
     const double dq = list_lattice_error(E);

@@ -1889,7 +1889,7 @@ template <class R> struct ListArgs {
     int cap;             // list capacity per particle (a multiple of 8)
     int narrow;          // 16-bit offsets, 8 per group (else 32-bit indices, 4 per group)
     const R* rl2t;       // squared list radius (rc + skin) per type pair; 0: no potential, never listed
-    R rl2max;            // the largest of them
+    R rl2max;            // squared reach of a list build's cells: the largest of them and the rounding of positions
     float thr2;          // squared displacement since the build above which the list check looks at a particle
     float cap2;          // squared displacement since the build that triggers a rebuild by itself
     int* hot;            // hot particles (moved more than sqrt(thr2)) of the last step, hot_max at most

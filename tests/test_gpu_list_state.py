@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from readdygpu_b200 import RdgpuError, _abi as A
-from readdygpu_b200.system import PairPotential
+from readdygpu_b200.system import System, ParticleType, PairPotential
 
 from .test_gpu_pairlist import same
 from .test_gpu_parity import Engine
@@ -137,3 +137,38 @@ def test_lists_that_outgrow_the_memory_in_a_step(mode):
         c.set_particles(xyz, types)
         c.step(30)
         same("f64", c.get_particles()[0], y)
+
+
+# Pairs a list radius of 9 nm apart on the z axis of a box of 7,000 nm whose
+# upper particle is the first FP32 position of its cell.  Seen from the lower
+# one, the distance to that cell rounds to more than 9 nm (1 + 5e-5).
+LIST_EDGE = [(6765.7744140625, 6774.7744140625), (6585.59423828125, 6594.59423828125),
+             (6864.87353515625, 6873.87353515625), (6405.4140625, 6414.4140625),
+             (6684.693359375, 6693.693359375), (6225.23388671875, 6234.23388671875)]
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+def test_lists_of_a_long_box_are_symmetric(prec):
+    """The pairs meet within one list: the upper particles move far enough to be
+    checked, the lower ones not, and the force must act on both."""
+    sys_ = System([ParticleType("A", 1e6, 3.0)],
+                  pair=[PairPotential(A.P2_HARMONIC, [(0, 0)], 1e4, "repulsive", r0=6.0)],
+                  kT=2.437, dt=1e-9, lo=(0, 0, 0), hi=(40, 40, 7000), periodic=(1, 1, 1))
+    xyz = np.array([(10.0 + k, 12.0, z) for k, p in enumerate(LIST_EDGE) for z in p])
+    types = np.zeros(len(xyz), np.int32)
+    move = np.zeros_like(xyz)
+    move[0::2, 2], move[1::2, 2] = 0.9, -2.35
+    out = []
+    for mode in ("cells", "list"):
+        with Engine(sys_, precision=prec, seed=2, neighbour_mode=mode, skin=3.0 if mode == "list" else 0.0) as e:
+            e.set_particles(xyz, types)
+            e.step_with_noise(move / np.sqrt(2.0 * 1e6 * 1e-9))
+            F, en = e.forces()
+            cnt, _ = e.neighbor_digest()
+            e.step(1)
+            m = e.metrics()
+            out.append((F, cnt, e.get_particles()[0]))
+    assert m["neighbour_mode"] == "list" and m["list_builds"] == 1      # the lists of the start
+    assert np.array_equal(out[0][1], np.ones(len(xyz))) and np.array_equal(out[1][1], out[0][1])
+    for a, b in ((out[0][0], out[1][0]), (out[0][2], out[1][2])):
+        same(prec, a, b)
