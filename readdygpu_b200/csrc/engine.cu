@@ -14,7 +14,6 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
-#include <unordered_set>
 #include <vector>
 
 #include "../../include/readdy_b200.h"
@@ -1912,7 +1911,7 @@ template <class R> int apply_edits_impl(Engine* E, const float* ed, long long co
 {
     const long long N = E->npart_tot;
     const int S = E->desc.n_types;
-    std::unordered_set<int> gone;
+    std::vector<bool> gone(N);           // by old id
     std::vector<int> del;
     std::vector<double> axyz;
     std::vector<int> atype;
@@ -1924,8 +1923,9 @@ template <class R> int apply_edits_impl(Engine* E, const float* ed, long long co
         const long long index = (long long)fi;
         const int newType = (int)ft;
         if (index != -1) {
-            if (index < 0 || index >= N || !gone.insert((int)index).second)
+            if (index < 0 || index >= N || gone[index])
                 return fail(E, RDGPU_ERR_ARG, "reaction entry " + std::to_string(r) + ": invalid or repeated gpu index");
+            gone[index] = true;
             del.push_back((int)index);
         }
         if (newType != -1) {
@@ -2013,7 +2013,7 @@ template <class R> int apply_edits_impl(Engine* E, const float* ed, long long co
         std::vector<int> nid(std::max<long long>(N, 1), -1);
         long long c = 0;
         for (long long i = 0; i < N; ++i)
-            if (!gone.count((int)i)) nid[i] = (int)c++;
+            if (!gone[i]) nid[i] = (int)c++;
         std::vector<int> ij, pot;
         for (size_t b = 0; b < E->bond_pot_h.size(); ++b) {
             const int i = nid[E->bond_ij_h[2 * b]], j = nid[E->bond_ij_h[2 * b + 1]];

@@ -132,3 +132,32 @@ def test_edits_need_single_system():
         e.set_particles(w.xyz, w.types, offsets=w.offsets)
         with pytest.raises(RuntimeError):
             e.apply_edits(edits((0,)))
+
+
+def test_edits_of_half_the_particles():
+    """10,000 deletions in any order with bonds on the survivors, and a
+    repetition among them, which is rejected."""
+    from readdygpu_b200.system import PairPotential
+    sys_, xyz, types = cfg1(20_000)
+    rng = np.random.default_rng(5)
+    gone = rng.permutation(20_000)[:10_000]
+    keep = np.setdiff1d(np.arange(20_000), gone)
+    ij = np.stack([keep[:-1:7], keep[1::7]], 1)[:1000]
+    ij = np.concatenate([ij, np.stack([gone[:50], keep[:50]], 1)])          # these go with their particles
+    new = np.full(20_000, -1)
+    new[keep] = np.arange(len(keep))
+    chain = [PairPotential(A.P2_HARMONIC, [], 5.0, "spring", r0=3.0)]
+    with Engine(sys_, precision="f64", seed=4) as e, Engine(sys_, precision="f64", seed=4) as f:
+        e.set_particles(xyz, types)
+        e.set_bonds(ij, np.zeros(len(ij), np.int32), chain)
+        with pytest.raises(RuntimeError):
+            e.apply_edits(edits(np.append(gone, gone[77])))
+        e.apply_edits(edits(gone, APP))
+        x, t = e.get_particles()
+        xe, te = expected(xyz, types, gone, APP)
+        np.testing.assert_array_equal(t, te)
+        assert np.abs(x - xe).max() <= 1e-12
+        f.set_particles(x, t)
+        f.set_bonds(new[ij[:1000]], np.zeros(1000, np.int32), chain)
+        (Fe, _), (Ff, _) = e.forces(), f.forces()
+        assert np.linalg.norm(Fe - Ff) <= 1e-12 * np.linalg.norm(Ff)
