@@ -155,6 +155,8 @@ struct rdgpu_engine {
     bool tuning = false;                 // inside tune(): its trials do not re-tune
     bool retune = false;                 // the lists outgrew their capacity: tune again
     int trial = 0;                       // an AUTO handle not tuned yet: see try_list
+    int trial_again = 0;                 // trials started over
+    long long trial_n = 0;               // the particles of the trial's first steps
     long long trial_steps = 0;
     double trial_s = 0.0, trial_cells = 0.0;
     RunCtl* run_ctl = nullptr;           // list_run_kernel: the control words of this launch and the next
@@ -1296,8 +1298,9 @@ template <class R> int do_steps_mode(Engine* E, long long nsteps, const double* 
 // The autotuner: times the cell walk and the pair list at a few skins on the
 // handle's own particles (graph_steps steps each after as many warm-up
 // steps, from a snapshot of the state that is restored afterwards) and keeps
-// the fastest.  The trajectory does not depend on the choice: the noise is
-// keyed by the step, and the FP32 forces are identical in both modes.
+// the fastest.  The trajectory does not depend on the choice (in FP64 to
+// rounding): the noise is keyed by the step, and the FP32 forces are identical
+// in both modes.
 template <class R> int tune(Engine* E)
 {
     E->tuned = true;
@@ -1406,13 +1409,41 @@ double trial_skin(const Engine* E)
 // calls have all been shorter than the tuner asks for.  The run itself is the
 // trial: kTrialCells steps of the cell walk and kTrialList steps of the pair
 // list are timed as they are made (each after an untimed chunk), and the
-// faster one stays.  No step is made twice and the trajectory does not depend
-// on the outcome.  7,919 particles (FP32C): 32.5 us a step with the cell walk,
+// faster one stays.  No step is made twice.  The outcome follows the host's
+// clock; the trajectory does not depend on it in FP32C, and in FP64 to rounding
+// only (the order of the sums).  7,919 particles (FP32C): 32.5 us a step with the cell walk,
 // 9 us with the list.
+//
+// A trial that meets another system before it ends (by more than a quarter of
+// the particles: an upload, or edits) would compare the cell walk of the one
+// with the list of the other, and starts over; one that ended on the cell walk
+// does so when the particle count has changed by more than a factor of two.
+// kTrialAgain times at most, so that a program that alternates between systems
+// gets an answer too.
 constexpr long long kTrialChunk = 16, kTrialCells = 16, kTrialList = 48;
+constexpr int kTrialAgain = 4;
+bool trial_due(const Engine* E)
+{
+    if (E->nb_req != RDGPU_NB_AUTO || E->tuned || E->graph_steps <= 0) return false;
+    if (E->trial < 5) return true;
+    const long long lo = std::min(E->npart_tot, E->trial_n), hi = std::max(E->npart_tot, E->trial_n);
+    return E->nb_mode == RDGPU_NB_CELLS && hi > 2 * lo && E->trial_again < kTrialAgain;
+}
 template <class R> int try_list(Engine* E, long long left)
 {
     const long long chunk = std::min(left, kTrialChunk);
+    const long long lo = std::min(E->npart_tot, E->trial_n), hi = std::max(E->npart_tot, E->trial_n);
+    if (E->trial == 5 || (E->trial > 0 && 4 * hi > 5 * lo && E->trial_again < kTrialAgain)) {
+        ++E->trial_again;
+        E->trial = 0;
+        if (E->nb_mode == RDGPU_NB_LIST)
+            if (const int rc = enter_cells<R>(E)) return rc;
+    }
+    if (E->trial == 0) {
+        E->trial_n = E->npart_tot;
+        E->trial_steps = 0;
+        E->trial_s = 0.0;
+    }
     if (E->trial == 2) {
         // the cell walk is timed: on to the list
         const double skin = trial_skin(E);
@@ -1459,8 +1490,7 @@ template <class R> int do_steps(Engine* E, long long nsteps, const double* noise
             int rc = tune<R>(E);
             if (rc) return rc;
         }
-        const bool trial = E->nb_req == RDGPU_NB_AUTO && !E->tuned && E->trial < 5 && E->graph_steps > 0 && !noise_d;
-        const int rc = trial ? try_list<R>(E, left) : do_steps_mode<R>(E, left, noise_d);
+        const int rc = trial_due(E) && !noise_d ? try_list<R>(E, left) : do_steps_mode<R>(E, left, noise_d);
         if (rc && rc != RDGPU_OK_CONTINUE) return rc;
     }
 }

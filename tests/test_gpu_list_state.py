@@ -172,3 +172,36 @@ def test_lists_of_a_long_box_are_symmetric(prec):
     assert np.array_equal(out[0][1], np.ones(len(xyz))) and np.array_equal(out[1][1], out[0][1])
     for a, b in ((out[0][0], out[1][0]), (out[0][2], out[1][2])):
         same(prec, a, b)
+
+
+@pytest.mark.parametrize("change", ["upload", "edits", "few edits"])
+@pytest.mark.parametrize("before", [40, 120])
+def test_trial_of_an_untuned_handle_meets_another_system(change, before):
+    """After 40 steps the trial is timing the list: another upload, or edits that
+    add 40 % of the particles, send it back to the cell walk; 4 % do not, and
+    after 120 steps it is over and its choice stays.  The trajectory is the cell
+    walk's throughout."""
+    sys_, xyz, types = plain(1000)
+    x2 = np.random.default_rng(2).uniform(0, sys_.hi[0], (5000, 3))
+    new = x2[:400 if change == "edits" else 40]
+    born = np.zeros((len(new), 6), np.float32)
+    born[:, 2:5], born[:, 5] = new, -1
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision="f32c", seed=4, neighbour_mode=mode) as e:
+            e.set_particles(xyz, types)
+            e.step(before)
+            first = e.metrics()["neighbour_mode"]
+            if change == "upload":
+                e.set_particles(x2, np.zeros(len(x2), np.int32))
+            else:
+                e.apply_edits(born)
+            e.step(8)
+            second = e.metrics()["neighbour_mode"]
+            e.step(90)
+            out.append(e.get_particles()[0])
+    if before == 40:
+        assert first == "list"
+    if first == "list":     # (the clock may have chosen the cell walk after 120 steps)
+        assert second == ("cells" if before == 40 and change != "few edits" else "list")
+    assert np.array_equal(out[0], out[1])
