@@ -1,13 +1,14 @@
 """The pair-list steps of an AUTO handle run in one launch per rdgpu_step call
 (list_run_kernel): the trajectory is the cell walk's, bit for bit in FP32C and
-to rounding in FP64, at the sizes where its shape changes (32-particle tiles,
-4 tiles per block, one block per SM, several blocks per SM), for every
-potential path, across rebuilds and whatever the split of the steps."""
+to rounding in FP64, at the sizes where its shape changes (one block per SM;
+up to 8 and 13 tiles of 32 particles per SM a warp keeps its tile, beyond that
+the warps draw tiles), for every potential path, across rebuilds and whatever
+the split of the steps."""
 import numpy as np
 import pytest
 
 from readdygpu_b200 import RdgpuError, _abi as A, configs
-from readdygpu_b200.system import System, ParticleType, PairPotential
+from readdygpu_b200.system import System, ParticleType, PairPotential, ExternalPotential
 
 from .test_gpu_pairlist import cluster_system, same
 from .test_gpu_parity import Engine, small_config2
@@ -317,3 +318,113 @@ def test_two_handles_in_two_threads():
         t.join()
     for seed in (1, 2):
         assert np.array_equal(alone[seed], together[seed])
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+@pytest.mark.parametrize("m", [4, 41])
+@pytest.mark.parametrize("gap", [-0.5, 0.3])
+def test_run_kernel_reports_a_failed_step(prec, m, gap):
+    """Particles on a grid (64: warps that keep their tile, 68,921: several
+    tiles per warp), tuned to the list, then eight pairs of them next to each
+    other: overlapping at once, or a few steps later.  Under an enormous force
+    constant the first overlap is a jump.  Its step, the state before it and
+    its forces are the cell walk's, and the next upload steps on."""
+    L = 14.0 * m
+    sys_ = System([ParticleType("A", 1e6, 1.5)],
+                  pair=[PairPotential(A.P2_HARMONIC, [(0, 0)], 1e12, "repulsive", r0=3.5)],
+                  kT=2.437, dt=1e-9, lo=(0, 0, 0), hi=(L, L, L), periodic=(1, 1, 1))
+    g = 14.0 * np.arange(m) + 7.0
+    xyz = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)
+    types = np.zeros(len(xyz), np.int32)
+    near = xyz.copy()
+    near[1:16:2] = near[0:16:2] + [3.5 + gap, 0, 0]
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision=prec, seed=5, neighbour_mode=mode) as e:
+            e.set_particles(xyz, types)
+            e.autotune()
+            e.set_particles(near, types)
+            assert mode == "cells" or e.metrics()["neighbour_mode"] == "list"
+            l0 = e.launch_count()
+            with pytest.raises(RdgpuError) as err:
+                e.step(100)
+            assert mode == "cells" or e.launch_count() == l0 + 1
+            assert err.value.code == -7
+            t = int(str(err.value).split("at step")[-1])
+            assert t == 0 if gap < 0 else 1 < t < 100
+            assert e.metrics()["step"] == t
+            got = [e.get_particles()[0], e.forces()[0]]
+            with pytest.raises(RdgpuError) as err:      # the same step again
+                e.step(3)
+            assert int(str(err.value).split("at step")[-1]) == t
+            got.append(e.get_particles()[0])
+            e.set_particles(xyz, types)
+            e.step(20)
+            got.append(e.get_particles()[0])
+            out.append((t, got))
+    assert out[0][0] == out[1][0]
+    for k, (a, b) in enumerate(zip(out[0][1], out[1][1])):
+        if prec == "f64" and k == 1:
+            assert np.linalg.norm(a - b) <= 1e-9 * np.linalg.norm(a)
+        else:
+            same(prec, a, b)
+
+
+@pytest.mark.parametrize("prec", ["f32c", "f64"])
+def test_run_kernel_overflow_regrows(prec):
+    """3,000 particles that a sphere's pull draws together within one call: lists
+    made for the dispersed state overflow inside list_run_kernel and grow."""
+    sys_ = System([ParticleType("A", 1e6, 1.0), ParticleType("B", 1e6, 1.0)],
+                  pair=[PairPotential(A.P2_HARMONIC, [(0, 0), (0, 1), (1, 1)], 0.01, "repulsive", r0=3.0)],
+                  external=[ExternalPotential(A.P1_SPHERE, [1], 100.0, "attractive", center=(40, 40, 40), radius=3.0)],
+                  kT=2.437, dt=1e-9, lo=(0, 0, 0), hi=(80, 80, 80), periodic=(1, 1, 1))
+    n = 3000
+    xyz = np.random.default_rng(3).uniform(0, 80, (n, 3))
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision=prec, seed=5, neighbour_mode=mode) as e:
+            e.set_particles(xyz, np.zeros(n, np.int32))     # type A is not drawn
+            e.autotune()
+            e.set_particles(xyz, np.ones(n, np.int32))
+            m0 = e.metrics()
+            e.step(100)
+            m1 = e.metrics()
+            e.step(30)
+            out.append(e.get_particles()[0])
+    assert m0["neighbour_mode"] == m1["neighbour_mode"] == "list"
+    assert m1["list_capacity"] > m0["list_capacity"] and m1["step"] == 100
+    same(prec, out[0], out[1])
+
+
+@pytest.mark.parametrize("system", ["slab", "mixed", "batch"])
+def test_fp32_diagnostics_over_the_list(oracle, system):
+    """FP32C, a running AUTO handle: forces, energy and neighbour sets over its
+    lists (32-bit entries, several terms per pair, a batch) are those of a cell
+    walk that made the same steps: forces and sets to the bit, the energy, which
+    the cells sum in FP32, to its rounding; and the oracle's."""
+    boxes = offsets = None
+    if system == "slab":
+        sys_, xyz, types, width = slab()
+    elif system == "mixed":
+        sys_, xyz, types = small_config2(3000)
+        width = 2
+    else:
+        w = configs.config4(n_systems=12, nmin=200, nmax=3000)
+        sys_, xyz, types, boxes, offsets, width = w.system, w.xyz, w.types, w.boxes, w.offsets, 2
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision="f32c", seed=3, boxes=boxes, neighbour_mode=mode) as e:
+            e.set_particles(xyz, types, offsets=offsets)
+            e.autotune()
+            e.step(37)
+            m = e.metrics()
+            out.append((e.get_particles()[0], *e.forces(), *e.neighbor_digest(), m["energy"]))
+    assert m["neighbour_mode"] == "list" and m["list_entry_bytes"] == width
+    (x, F, en, cnt, h, en2), (xl, Fl, enl, cntl, hl, enl2) = out
+    assert np.array_equal(x, xl) and np.array_equal(F, Fl) and np.array_equal(cnt, cntl) and np.array_equal(h, hl)
+    assert enl == enl2 and abs(enl - en) <= 1e-5 * abs(en)
+    if system == "mixed":
+        hi, comp = oracle.to_rel_f32(sys_.to_desc(), xl)
+        Fo, eo = oracle.forces_f64(sys_.to_desc(), hi.astype(np.float64).reshape(-1, 3), types)
+        assert abs(enl - eo) <= 1e-5 * abs(eo)
+        assert np.linalg.norm(Fl - Fo) <= 1e-5 * np.linalg.norm(Fo)
