@@ -131,9 +131,13 @@ typedef struct {
    more than about skin since the last build; after every step the particles
    that moved more than about skin/2 have their current neighbourhood
    checked against the list.  The pair set and the FP32 forces are identical
-   to CELLS.  AUTO starts with CELLS, times some 30 steps of it and 50 of LIST
-   (at a skin estimated from the diffusion constants) as it makes them and
-   keeps the faster; at the first rdgpu_step of >= 4 x graph_steps steps, or in
+   to CELLS.  AUTO starts with CELLS, times at least 16 steps of it and 48 of
+   LIST (at a skin estimated from the diffusion constants) as it makes them,
+   each after up to 16 untimed ones, and keeps the faster, which follows the
+   host's clock (FP64 results then differ by the rounding of sums made in
+   another order); it starts over, four times at most, when the particle count
+   changes by more than a quarter before it is done, or by more than a factor
+   of two after it kept CELLS; at the first rdgpu_step of >= 4 x graph_steps steps, or in
    rdgpu_autotune, it times CELLS and LIST at skins of 0.1 .. 0.5 x rc_max on
    the handle's particles and keeps the fastest; the pair-list steps of an AUTO
    handle run many to a kernel launch, those of a LIST handle launch by launch

@@ -8,10 +8,15 @@
 // and a conditional graph node per step), 8 to 40 us of every step went to
 // launch gaps, the check's own launch and the conditional node: more than the
 // step itself up to about a million particles.  Per step, launch by launch
-// and in one launch (tuned, steps of a 100-step frame): 1,000 particles FP64
-// 19.7 and 10.0 us, 20,000 FP64 22.2 and 11.6, 250,000 (vesicle, FP32C) 56.7
-// and 47.1, 370,000 FP64 in 64 systems 54.5 and 38.0, 2.9 M in 512 systems
-// 158 and 152 (there the step and the list build are bound by issue).
+// and in one launch (tuned, calls of 100 steps, rebuilds and the host's wait
+// included): 1,000 particles FP64 20.5 and 5.8 us, 20,000 FP64 23.0 and 6.7,
+// 250,000 (vesicle, FP32C) 52.4 and 30.5, 370,000 FP64 in 64 systems 53.5 and
+// 33.2, 2.9 M in 512 systems 152 and 126 (there the step and the list build
+// are bound by issue).
+//
+// The before-and-after figures at the parts below are of the builds in which
+// each part was taken (skin 1.4), one after the other: they price the part,
+// and are not the times of the kernel as it stands.
 #pragma once
 #include "engine_kernels.cuh"
 
