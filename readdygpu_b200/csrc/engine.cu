@@ -1342,6 +1342,10 @@ template <class R> int tune(Engine* E)
         if (rc) break;
         // the snapshot is sorted for the grid it was taken on; re-sort on the candidate's
         rc = skins[c] > 0.0 ? enter_list<R>(E, skins[c]) : (E->nb_mode = RDGPU_NB_LIST, enter_cells<R>(E));
+        if (rc == RDGPU_ERR_NOMEM && skins[c] > 0.0) {
+            rc = RDGPU_OK;      // its lists do not fit
+            continue;
+        }
         if (rc) break;
         // a trial that fails (the dynamics itself, e.g. a particle leaving the
         // box) disqualifies the candidate; the real run reports the failure

@@ -94,6 +94,20 @@ def test_untuned_handle_whose_lists_do_not_fit_keeps_the_cell_walk():
     assert np.array_equal(out[0], out[1])
 
 
+def test_tuner_passes_over_lists_that_do_not_fit():
+    sys_, _, packed, types = clot()
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision="f32c", seed=2, neighbour_mode=mode) as e:
+            e.set_particles(packed, types)
+            e.autotune()
+            e.step(5)
+            m = e.metrics()
+            out.append(e.get_particles()[0])
+    assert m["neighbour_mode"] == "cells" and m["step"] == 5
+    assert np.array_equal(out[0], out[1])
+
+
 @pytest.mark.parametrize("mode", ["list", "auto"])
 def test_lists_that_outgrow_the_memory_in_a_step(mode):
     """The step that draws the particles together stands and its lists are
