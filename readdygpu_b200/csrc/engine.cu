@@ -1150,6 +1150,17 @@ template <class R> int enter_cells(Engine* E)
     return RDGPU_OK;
 }
 
+// rc of a call that needed pair lists: an AUTO handle whose lists do not fit the
+// device memory goes on with the cell walk (until it is tuned again)
+template <class R> int lists_or_cells(Engine* E, int rc)
+{
+    if (rc != RDGPU_ERR_NOMEM || E->nb_req != RDGPU_NB_AUTO || E->nb_mode != RDGPU_NB_LIST) return rc;
+    E->retune = E->tuned;
+    E->trial = 5;
+    E->trial_n = E->npart_tot;
+    return enter_cells<R>(E);
+}
+
 // the pair-list graph of n steps (captured on first use)
 template <class R> int capture_list_graph(Engine* E, int n, cudaGraphExec_t* out)
 {
@@ -1455,8 +1466,7 @@ template <class R> int try_list(Engine* E, long long left)
         if (list_eligible(E, skin)) {
             const int rc = enter_list<R>(E, skin);
             if (rc == RDGPU_OK) E->trial = 3;
-            else if (rc != RDGPU_ERR_NOMEM) return rc;
-            else if (const int rn = enter_cells<R>(E)) return rn;
+            else if (const int rn = lists_or_cells<R>(E, rc)) return rn;
         }
         E->trial_steps = 0;
         E->trial_s = 0.0;
@@ -1494,7 +1504,8 @@ template <class R> int do_steps(Engine* E, long long nsteps, const double* noise
             int rc = tune<R>(E);
             if (rc) return rc;
         }
-        const int rc = trial_due(E) && !noise_d ? try_list<R>(E, left) : do_steps_mode<R>(E, left, noise_d);
+        const int rc = lists_or_cells<R>(
+            E, trial_due(E) && !noise_d ? try_list<R>(E, left) : do_steps_mode<R>(E, left, noise_d));
         if (rc && rc != RDGPU_OK_CONTINUE) return rc;
     }
 }
@@ -1892,6 +1903,16 @@ template <class R, class In> int set_particles_impl(Engine* E, const long long* 
     E->part_off = off;
     if (list_mode) {
         rc = resort<R>(E, true, one);
+        if (rc == RDGPU_ERR_NOMEM && one) {
+            // (the input has not been looked at if there was no storage to begin with)
+            int ef = 0;
+            if (cudaStreamSynchronize(E->stream) != cudaSuccess ||
+                cudaMemcpy(&ef, E->err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+                rc = fail(E, RDGPU_ERR_CUDA, "upload check failed");
+            else if (ef & EF_BADINPUT)
+                rc = fail(E, RDGPU_ERR_ARG, kBadInput);
+        }
+        rc = lists_or_cells<R>(E, rc);
         if (rc) { E->part_off.clear(); return rc; }
     }
     return RDGPU_OK;
@@ -2066,7 +2087,7 @@ template <class R> int apply_edits_impl(Engine* E, const float* ed, long long co
         if (rc) return rc;
     }
     if (E->nb_mode == RDGPU_NB_LIST) {
-        rc = resort<R>(E, true);
+        rc = lists_or_cells<R>(E, resort<R>(E, true));
         if (rc) { E->part_off.clear(); return rc; }
     }
     return RDGPU_OK;
@@ -2115,7 +2136,9 @@ template <class R> int sync_types(Engine* E)
 // once; missing ones, which the walk can do without, by the next step.
 template <class R> int fresh_cells(Engine* E)
 {
-    return E->nb_mode == RDGPU_NB_LIST ? resort<R>(E, E->list_valid) : RDGPU_OK;
+    if (E->nb_mode != RDGPU_NB_LIST) return RDGPU_OK;
+    const int rc = resort<R>(E, E->list_valid);
+    return rc == RDGPU_ERR_NOMEM ? resort<R>(E, false) : rc;
 }
 
 // forces and energies (MODE 1) or neighbour digest (MODE 2) of the current

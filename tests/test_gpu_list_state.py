@@ -1,7 +1,8 @@
 """Handles in pair-list mode whose lists are gone.  After a rejected edit that had
 grown the buffers, steps, forces, energies, neighbour sets and RDF frames are
 those of a handle that never saw the edit.  When the lists outgrow the device
-memory, the call that needs them says so and the rest goes on."""
+memory, an AUTO handle goes on with the cell walk, and one that asked for lists
+says so and can still be read and evaluated."""
 import numpy as np
 import pytest
 
@@ -108,21 +109,22 @@ def test_tuner_passes_over_lists_that_do_not_fit():
     assert np.array_equal(out[0], out[1])
 
 
-@pytest.mark.parametrize("mode", ["list", "auto"])
-def test_lists_that_outgrow_the_memory_in_a_step(mode):
-    """The step that draws the particles together stands and its lists are
-    refused; the state can be read and evaluated, steps are refused as long as
-    it lasts, and the next upload steps on."""
+def gather(e, xyz, packed, types):
+    """One step with the noise that takes every particle from xyz to packed."""
+    b = np.sqrt(2.0 * np.array([t.D for t in e.system.types])[types] * e.system.dt)[:, None]
+    e.step_with_noise((packed - xyz) / b)
+
+
+def test_lists_that_outgrow_the_memory_in_a_step():
+    """A handle that asks for lists: the step that draws the particles together
+    stands and its lists are refused; the state can be read and evaluated, steps
+    are refused as long as it lasts, and the next upload steps on."""
     sys_, xyz, packed, types = clot()
-    n = len(xyz)
-    b = np.sqrt(2.0 * np.array([t.D for t in sys_.types])[types] * sys_.dt)[:, None]
-    with Engine(sys_, precision="f64", seed=2, neighbour_mode=mode, skin=1.0 if mode == "list" else 0.0) as e:
+    with Engine(sys_, precision="f64", seed=2, neighbour_mode="list", skin=1.0) as e:
         e.set_particles(xyz, types)
-        if mode == "auto":
-            e.autotune()
         assert e.metrics()["neighbour_mode"] == "list"
         with pytest.raises(RdgpuError) as err:
-            e.step_with_noise((packed - xyz) / b)
+            gather(e, xyz, packed, types)
         assert err.value.code == -6
         m = e.metrics()
         assert m["step"] == 1 and m["neighbour_mode"] == "list"
@@ -151,6 +153,47 @@ def test_lists_that_outgrow_the_memory_in_a_step(mode):
         c.set_particles(xyz, types)
         c.step(30)
         same("f64", c.get_particles()[0], y)
+
+
+@pytest.mark.parametrize("how", ["step", "upload", "edits"])
+@pytest.mark.parametrize("tuned", [False, True])
+def test_auto_handle_whose_lists_outgrow_the_memory(how, tuned):
+    """An AUTO handle in pair-list mode goes on with the cell walk: through the
+    step that draws the particles together, the upload of the clot (a bad
+    coordinate is still refused) or the edits that add it."""
+    sys_, xyz, packed, types = clot()
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision="f32c", seed=2, neighbour_mode=mode) as e:
+            e.set_particles(xyz, types)
+            if tuned:
+                e.autotune()
+            else:
+                e.step(100)
+                e.set_particles(xyz, types)
+            first = e.metrics()["neighbour_mode"]
+            if how == "step":
+                gather(e, xyz, packed, types)
+            elif how == "upload":
+                bad = packed.copy()
+                bad[3, 1] = np.nan
+                with pytest.raises(RdgpuError) as err:
+                    e.set_particles(bad, types)
+                assert err.value.code == -1
+                e.set_particles(packed, types)
+            else:
+                m = 25_000
+                rows = np.zeros((m, 6), np.float32)
+                rows[:, 2:5], rows[:, 5] = packed[:m], -1
+                e.apply_edits(rows)
+            e.step(10)
+            last = e.metrics()
+            F, en = e.forces()
+            out.append((e.get_particles()[0], F))
+    assert first == "list" and last["neighbour_mode"] == "cells"
+    assert last["step"] == (11 if how == "step" else 10)
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
 
 
 # Pairs a list radius of 9 nm apart on the z axis of a box of 7,000 nm whose
