@@ -747,15 +747,17 @@ bool list_eligible(Engine* E, double skin)
     return true;
 }
 
+// entries of a list, at most: whole groups below the list head's count field
+constexpr int kListMost = 65528;
+
 // list storage for cap entries per particle (wide: 32-bit entries)
 int ensure_list(Engine* E, int cap, bool wide)
 {
     const long long stride = std::max<long long>(E->cap_particles, 1);
     if (cap <= E->list_cap && stride == E->list_stride && wide == E->list_wide && E->nbr) return RDGPU_OK;
     // whole groups of 8 entries (one int4 narrow, two wide): the step kernel
-    // requests the first 8 entries before it knows the list length; at most
-    // 2^16 - 1 (the list head's count field)
-    cap = std::min((std::max(std::max(cap, E->list_cap), 8) + 7) & ~7, 65528);
+    // requests the first 8 entries before it knows the list length
+    cap = std::min((std::max(std::max(cap, E->list_cap), 8) + 7) & ~7, kListMost);
     drop_graph_map(E->lgraphs);
     dfree(E->nbr); dfree(E->head); dfree(E->hot);
     E->list_valid = false;
@@ -787,6 +789,10 @@ int ensure_list_after(Engine* E, int ef)
 {
     // taken note of: the scans of other calls (an RDF frame) stop at a set flag
     CK(cudaMemsetAsync(E->err, 0, sizeof(int), E->stream));
+    if ((ef & EF_LISTOVF) && E->pinned_ctl->maxcnt > kListMost) {
+        E->list_valid = false;
+        return fail(E, RDGPU_ERR_NOMEM, "a pair list of " + std::to_string(E->pinned_ctl->maxcnt) + " entries");
+    }
     const int cap = (ef & EF_LISTOVF) ? list_regrow_cap(E) : E->list_cap;
     return ensure_list(E, cap, E->list_wide || (ef & EF_LISTWIDE) != 0);
 }

@@ -95,6 +95,29 @@ def test_untuned_handle_whose_lists_do_not_fit_keeps_the_cell_walk():
     assert np.array_equal(out[0], out[1])
 
 
+@pytest.mark.parametrize("tuned", [False, True])
+def test_lists_longer_than_their_heads_can_count(tuned):
+    """70,000 particles in a cube of edge 1: more partners than the 16-bit count
+    of a list head takes.  AUTO handles keep the cell walk, a handle that asks
+    for lists is refused its upload."""
+    sys_, _, packed, types = clot(71_000, 70_000)
+    out = []
+    for mode in ("cells", "auto"):
+        with Engine(sys_, precision="f32c", seed=2, neighbour_mode=mode) as e:
+            e.set_particles(packed, types)
+            if tuned:
+                e.autotune()
+            e.step(40)
+            m = e.metrics()
+            out.append(e.get_particles()[0])
+    assert m["neighbour_mode"] == "cells" and m["step"] == 40
+    assert np.array_equal(out[0], out[1])
+    with Engine(sys_, precision="f32c", neighbour_mode="list", skin=1.0) as e:
+        with pytest.raises(RdgpuError) as err:
+            e.set_particles(packed, types)
+        assert err.value.code == -6 and "70" in str(err.value)
+
+
 def test_tuner_passes_over_lists_that_do_not_fit():
     sys_, _, packed, types = clot()
     out = []
