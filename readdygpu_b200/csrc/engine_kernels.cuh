@@ -2353,7 +2353,8 @@ template <class R> struct ListCell {
 // Squared minimum-image distances of the list build: d = (xi - xj) - k L with
 // k = rint((xi - xj) / L), each operation rounded once.  Swapping i and j
 // negates every intermediate, so the test of a pair is the same from both
-// sides and j is in i's list exactly when i is in j's.
+// sides.  Both look into each other's cells (ListArgs::rl2max allows for the
+// rounding that chooses them), so j is in i's list exactly when i is in j's.
 template <class R> struct PairSym;
 template <> struct PairSym<float> {
     f32x2 xy, il_xy, nl_xy;
