@@ -139,7 +139,8 @@ typedef struct {
    changes by more than a quarter before it is done, or by more than a factor
    of two after it kept CELLS; at the first rdgpu_step of >= 4 x graph_steps steps, or in
    rdgpu_autotune, it times CELLS and LIST at skins of 0.1 .. 0.5 x rc_max on
-   the handle's particles and keeps the fastest; the pair-list steps of an AUTO
+   the handle's particles and keeps the fastest; where its lists do not fit the
+   device memory it goes on with CELLS; the pair-list steps of an AUTO
    handle run many to a kernel launch, those of a LIST handle launch by launch
    in captured graphs.  Energies, forces and
    digests in LIST mode are evaluated over the list, which holds every pair
